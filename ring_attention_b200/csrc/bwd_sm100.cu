@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
   const int hh = bh % p.h, bb = bh / p.h;
   const uint32_t kinds = p.mod.kinds;
   const bool masked = (kinds & kMetaKinds) != 0;  // the tile summaries are read
-  const bool dense = (kinds & RA_MOD_DENSE) != 0;  // every tile takes the in-TMEM pass (it adds the bias tile)
+  const bool dense = (kinds & RA_MOD_DENSE) != 0;  // every tile takes the in-TMEM pass that adds the bias tile
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < NUM_BARS; ++i) {
@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
     int32_t hit_pos0 = 0;   // pos0 of the tile the last call returned
   };
   auto next_active = [&](Window& w, int i) -> int {
-    if (!masked) return i < P.n_q_tiles ? (i | (dense ? kMixedBit : 0)) : P.n_q_tiles;
+    if (!masked) return i < P.n_q_tiles ? i : P.n_q_tiles;
     while (i < P.n_q_tiles) {
       if (i < w.base || i >= w.base + 32) {
         w.base = i;
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
         const int first = __ffs(vote) - 1;
         const int c = __shfl_sync(0xffffffffu, w.cls, first);
         w.hit_pos0 = __shfl_sync(0xffffffffu, w.pos0, first);
-        return (w.base + first) | (((c & 3) == 2 || dense) ? kMixedBit : 0) | ((c & 4) ? kContigBit : 0);
+        return (w.base + first) | ((c & 3) == 2 ? kMixedBit : 0) | ((c & 4) ? kContigBit : 0);
       }
       i = w.base + 32;
     }
@@ -499,23 +499,25 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
         // ---- P^T = exp2(S^T * scale2 - L * log2e) of tile k on this warpgroup's 64 query columns
         const int n = k, s = n & 1, i = i_cur;
         const bool need_mask = (e_cur & kMixedBit) != 0;
-        // ALiBi over a tile of contiguous query positions with nothing masked is two FMAs per
-        // score in registers; every other ALiBi tile takes the in-TMEM pass below
-        const bool alibi_inline = alibi && !need_mask && (e_cur & kContigBit) != 0;
+        // ALiBi over a tile of contiguous query positions is two FMAs per score in registers, over
+        // scattered ones it takes the in-TMEM pass below
+        const bool alibi_inline = alibi && (e_cur & kContigBit) != 0;
+        const int64_t q0 = (int64_t)bb * p.lq + (int64_t)i * kTileRows + g * 64;
+        uint32_t vis[2];
+        if (need_mask)  // found while the scores are on their way
+          visible_columns<false>(vis, kinds, p.mod.window, kpos, kseg, kpre, p.mod.q_pos + q0, p.mod.q_seg + q0,
+                                 p.mod.q_pre + q0, q0_cur + g * 64, (e_cur & kContigBit) != 0);
         if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[Q_FULL0 + s], (n >> 1) & 1, abort_flag, P.status, kStBwdCompute)))) break;
         const float4* Ls = reinterpret_cast<const float4*>(sL + s * kTileRows + g * 64);
         if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[S_FULL], n & 1, abort_flag, P.status, kStBwdCompute)))) break;
         tc_fence_after();
-        if (need_mask || (alibi && !alibi_inline)) {  // tiles that mix visible and masked pairs, ALiBi over scattered positions
-          const int64_t q0 = (int64_t)bb * p.lq + (int64_t)i * kTileRows + g * 64;
-          fixup_scores_tmem<false>(tmem_S + lane_off + g * 64, 64, need_mask ? kinds : (kinds & RA_MOD_ALIBI),
-                                   p.mod.window, alibi_over_scale, kpos, kseg, kpre,
-                                   p.mod.q_pos ? p.mod.q_pos + q0 : nullptr, p.mod.q_seg ? p.mod.q_seg + q0 : nullptr,
-                                   p.mod.q_pre ? p.mod.q_pre + q0 : nullptr, q0_cur + g * 64, (e_cur & kContigBit) != 0,
-                                   dense ? p.mod.bias + (int64_t)bb * p.mod.bsb + (int64_t)hh * p.mod.bsh +
-                                               ((int64_t)i * kTileRows + g * 64) * p.mod.bsq + kv_row
-                                         : nullptr,
-                                   p.mod.bsq, 1.f / p.scale);
+        if (dense || (alibi && !alibi_inline)) {
+          bias_scores_tmem<false>(tmem_S + lane_off + g * 64, 64, alibi && !alibi_inline, alibi_over_scale, kpos,
+                                  p.mod.q_pos + q0,
+                                  dense ? p.mod.bias + (int64_t)bb * p.mod.bsb + (int64_t)hh * p.mod.bsh +
+                                              ((int64_t)i * kTileRows + g * 64) * p.mod.bsq + kv_row
+                                        : nullptr,
+                                  p.mod.bsq, 1.f / p.scale);
         }
         tmem_ld32(tmem_S + lane_off + g * 64, sv[0]);
         tmem_ld32(tmem_S + lane_off + g * 64 + 32, sv[1]);
@@ -529,6 +531,11 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
           for (int c = 0; c < 64; ++c)
             sv[c >> 5][c & 31] = __float_as_uint(fmaf(-slope2, (float)c, fmaf(__uint_as_float(sv[c >> 5][c & 31]), scale2, rr)));
           sc = 1.f;
+        }
+        if (need_mask) {  // a tile that mixes visible and masked pairs
+#pragma unroll
+          for (int c = 0; c < 64; ++c)
+            if (!((vis[c >> 5] >> (c & 31)) & 1u)) sv[c >> 5][c & 31] = 0xff800000u;  // -inf
         }
         if (dense) {
           // With a dense bias tile the reference's arithmetic is kept as it is (ring.py:146): a row

@@ -47,6 +47,12 @@ struct FwdTcParams {
   unsigned int* status;
 };
 
+// An entry of a CTA's list of K/V tiles: the tile's index, "query tile t sees something of it" at
+// kVisible << t, "and not all of it" at kMixed << t, "its positions are contiguous" at kContig.
+constexpr int kTileBits = 12;
+constexpr uint32_t kTileIdx = (1u << kTileBits) - 1, kVisible = 1u << 12, kMixed = 1u << 14, kContig = 1u << 16;
+static_assert(kMaxTiles <= (1 << kTileBits), "tile index does not fit a list entry");
+
 enum Bar {
   Q_FULL0 = 0, Q_FULL1, K_FULL0, K_FULL1, K_EMPTY0, K_EMPTY1, V_FULL0, V_FULL1, V_EMPTY0, V_EMPTY1,
   S_FULL0, S_FULL1, P_FULL0, P_FULL1, O_FULL, NUM_BARS
@@ -62,8 +68,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
   uint8_t* sQ = smem;
   uint8_t* sK = sQ + 2 * TILE_BYTES;
   uint8_t* sV = sK + 2 * TILE_BYTES;
-  uint16_t* list = reinterpret_cast<uint16_t*>(sV + 2 * TILE_BYTES);
-  uint8_t* codes = reinterpret_cast<uint8_t*>(list + kMaxTiles);  // [kMaxTiles] class of each K/V tile
+  uint32_t* list = reinterpret_cast<uint32_t*>(sV + 2 * TILE_BYTES);  // the K/V tiles this CTA visits
+  uint8_t* codes = reinterpret_cast<uint8_t*>(list + kMaxTiles);       // [kMaxTiles] class of each K/V tile
   uint64_t* bars = reinterpret_cast<uint64_t*>(codes + kMaxTiles);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NUM_BARS);
   volatile uint32_t* abort_flag = tmem_slot + 1;
@@ -93,12 +99,13 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
-  // List of K/V tiles this CTA visits: index in bits 0-11, "query tile t needs mask arithmetic
-  // on it" in bit 12+t, "the tile's positions are contiguous" in bit 14.  Tiles masked for both
-  // query tiles are left out.  Every thread classifies its share of the tiles (one round of
-  // loads for up to 320 tiles), then warp 0 compacts the classes in order.
+  // List of K/V tiles this CTA visits (index and class bits, see kTileIdx ...).  Tiles masked for
+  // both query tiles are left out; a tile masked for one of them is visited for the other only.
+  // Every thread classifies its share of the tiles (one round of loads for up to 320 tiles), then
+  // warp 0 compacts the classes in order.
   const bool masked = (kinds & kMetaKinds) != 0;
-  const bool dense = (kinds & RA_MOD_DENSE) != 0;  // every visited tile takes the in-TMEM pass (it adds the bias tile)
+  const bool dense = (kinds & RA_MOD_DENSE) != 0;
+  const uint32_t all_visible = ntile == 2 ? (kVisible << 0) | (kVisible << 1) : kVisible;
   if (masked) {
     const TileMeta mq0 = P.meta_q[bb * P.n_q_tiles + qt0];
     const TileMeta mq1 = P.meta_q[bb * P.n_q_tiles + qt0 + (ntile - 1)];
@@ -106,8 +113,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
       const TileMeta mk = P.meta_kv[bb * P.n_kv_tiles + j];
       const int c0 = classify_tiles(kinds, p.mod.window, mq0, mk);
       const int c1 = ntile == 2 ? classify_tiles(kinds, p.mod.window, mq1, mk) : 0;
-      const uint32_t code = ((c0 != 1 || dense) ? 1u : 0u) | ((c1 != 1 || dense) ? 2u : 0u) | (mk.pos_contig ? 4u : 0u);
-      codes[j] = ((c0 != 0) || (c1 != 0)) ? (uint8_t)(0x80u | code) : (uint8_t)0;  // bit 7: visited
+      const uint32_t code = (c0 != 0 ? kVisible : 0u) | (c1 != 0 ? kVisible << 1 : 0u) | (c0 == 2 ? kMixed : 0u) |
+                            (c1 == 2 ? kMixed << 1 : 0u) | (mk.pos_contig ? kContig : 0u);
+      codes[j] = (uint8_t)(code >> kTileBits);
     }
     __syncthreads();
   }
@@ -116,13 +124,13 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
     for (int base = 0; base < P.n_kv_tiles; base += 32) {
       const int j = base + lane;
       bool active = j < P.n_kv_tiles;
-      uint32_t code = dense ? 3u : 0u;
+      uint32_t code = all_visible;
       if (active && masked) {
-        code = codes[j] & 0x7u;
-        active = (codes[j] & 0x80u) != 0;
+        code = (uint32_t)codes[j] << kTileBits;
+        active = (code & all_visible) != 0;
       }
       const uint32_t vote = __ballot_sync(0xffffffffu, active);
-      if (active) list[cnt + __popc(vote & ((1u << lane) - 1))] = (uint16_t)(j | (code << 12));
+      if (active) list[cnt + __popc(vote & ((1u << lane) - 1))] = (uint32_t)j | code;
       cnt += __popc(vote);
     }
     // ALiBi makes the scores grow towards the query's own position: visiting the K/V tiles in
@@ -131,7 +139,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
     if ((kinds & RA_MOD_ALIBI) && !(kinds & RA_MOD_DENSE)) {
       __syncwarp();
       for (int i = lane; i < cnt / 2; i += 32) {
-        const uint16_t a = list[i], z = list[cnt - 1 - i];
+        const uint32_t a = list[i], z = list[cnt - 1 - i];
         list[i] = z;
         list[cnt - 1 - i] = a;
       }
@@ -159,7 +167,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
                       (qt0 + t) * kTileRows, bb);
       }
       for (int i = 0; i < count; ++i) {
-        const int j = list[i] & 0xFFF, s = i & 1;
+        const int j = list[i] & kTileIdx, s = i & 1;
         const uint32_t ph = (i >> 1) & 1;
         if (!mbar_wait(&bars[K_EMPTY0 + s], ph ^ 1, abort_flag, P.status, kStFwdProducer)) break;
         mbar_arrive_expect_tx(&bars[K_FULL0 + s], TILE_BYTES);
@@ -204,24 +212,29 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
       if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&bars[K_FULL0], 0, abort_flag, P.status, kStFwdMma));
       if (ok) {
         tc_fence_after();
-        for (int t = 0; t < ntile; ++t) issue_s(t, 0);
+        for (int t = 0; t < ntile; ++t)
+          if (list[0] & (kVisible << t)) issue_s(t, 0);
         tc_commit_warp(&bars[K_EMPTY0]);
       }
+      int done[2] = {0, 0};  // K/V tiles each query tile has been through
       for (int i = 0; i < count && ok; ++i) {
         const int s = i & 1, sn = (i + 1) & 1;
         const uint32_t ph = (i >> 1) & 1, phn = ((i + 1) >> 1) & 1;
         const bool has_next = i + 1 < count;
+        const uint32_t cur = list[i], nxt = has_next ? list[i + 1] : 0u;
         if (has_next && !(ok = __all_sync(0xffffffffu, mbar_wait(&bars[K_FULL0 + sn], phn, abort_flag, P.status, kStFwdMma)))) break;
         if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[V_FULL0 + s], ph, abort_flag, P.status, kStFwdMma)))) break;
-        for (int t = 0; t < ntile; ++t) {
-          if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[P_FULL0 + t], i & 1, abort_flag, P.status, kStFwdMma)))) break;
-          tc_fence_after();
-          issue_pv(t, s, i == 0);
-          if (t == ntile - 1) tc_commit_warp(&bars[V_EMPTY0 + s]);
-          if (has_next) {
-            issue_s(t, sn);
-            if (t == ntile - 1) tc_commit_warp(&bars[K_EMPTY0 + sn]);
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          if (cur & (kVisible << t)) {
+            if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[P_FULL0 + t], done[t] & 1, abort_flag, P.status, kStFwdMma)))) break;
+            tc_fence_after();
+            issue_pv(t, s, done[t] == 0);
+            ++done[t];
           }
+          if (t == ntile - 1) tc_commit_warp(&bars[V_EMPTY0 + s]);
+          if (nxt & (kVisible << t)) issue_s(t, sn);
+          if (has_next && t == ntile - 1) tc_commit_warp(&bars[K_EMPTY0 + sn]);
         }
       }
       if (ok) tc_commit_warp(&bars[O_FULL]);
@@ -253,28 +266,33 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
     const float slope2 = alibi ? p.mod.slopes[hh] * kLog2e : 0.f;
     // first position of the K/V tile the loop is about to visit, read one tile ahead
     const bool has_pos = p.mod.kv_pos != nullptr;
-    int32_t k0_next = (has_pos && count > 0) ? p.mod.kv_pos[(int64_t)bb * p.lk + (int64_t)(list[0] & 0xFFF) * kTileRows] : 0;
+    int32_t k0_next = (has_pos && count > 0) ? p.mod.kv_pos[(int64_t)bb * p.lk + (int64_t)(list[0] & kTileIdx) * kTileRows] : 0;
+    int done = 0;  // K/V tiles this query tile has been through
     for (int i = 0; i < count; ++i) {
-      const int j = list[i] & 0xFFF;
-      const bool need_mask = ((list[i] >> (12 + t)) & 1) != 0;
-      // ALiBi over a tile of contiguous key positions with nothing masked is two FMAs per score
-      // in registers; every other ALiBi tile takes the in-TMEM pass below
-      const bool kv_contig = ((list[i] >> 14) & 1) != 0;
-      const bool alibi_inline = alibi && !need_mask && kv_contig;
+      const uint32_t entry = list[i];
+      const int j = entry & kTileIdx;
+      const bool need_mask = (entry & (kMixed << t)) != 0;
+      // ALiBi over a tile of contiguous key positions is two FMAs per score in registers, over
+      // scattered ones it takes the in-TMEM pass below
+      const bool kv_contig = (entry & kContig) != 0;
+      const bool alibi_inline = alibi && kv_contig;
       const int32_t k0 = k0_next;
-      if (has_pos && i + 1 < count) k0_next = p.mod.kv_pos[(int64_t)bb * p.lk + (int64_t)(list[i + 1] & 0xFFF) * kTileRows];
-      if (!(ok = mbar_wait(&bars[S_FULL0 + t], i & 1, abort_flag, P.status, kStFwdSoftmax))) break;
+      if (has_pos && i + 1 < count) k0_next = p.mod.kv_pos[(int64_t)bb * p.lk + (int64_t)(list[i + 1] & kTileIdx) * kTileRows];
+      if (!(entry & (kVisible << t))) continue;
+      const int64_t kv0 = (int64_t)bb * p.lk + (int64_t)j * kTileRows;
+      uint32_t vis[4];
+      if (need_mask)  // a tile that mixes visible and masked pairs: found while its scores are on their way
+        visible_columns<true>(vis, kinds, p.mod.window, qpos, qseg, qpre, p.mod.kv_pos + kv0, p.mod.kv_seg + kv0,
+                              p.mod.kv_pre + kv0, k0, kv_contig);
+      if (!(ok = mbar_wait(&bars[S_FULL0 + t], done & 1, abort_flag, P.status, kStFwdSoftmax))) break;
       tc_fence_after();
-      if (need_mask || (alibi && !alibi_inline)) {  // tiles that mix visible and masked pairs, ALiBi over scattered positions
-        const int64_t kv0 = (int64_t)bb * p.lk + (int64_t)j * kTileRows;
-        fixup_scores_tmem<true>(tmem_S[t] + lane_off, kTileRows, need_mask ? kinds : (kinds & RA_MOD_ALIBI),
-                                p.mod.window, alibi_over_scale, qpos, qseg, qpre,
-                                p.mod.kv_pos ? p.mod.kv_pos + kv0 : nullptr, p.mod.kv_seg ? p.mod.kv_seg + kv0 : nullptr,
-                                p.mod.kv_pre ? p.mod.kv_pre + kv0 : nullptr, k0, kv_contig,
-                                dense ? p.mod.bias + (int64_t)bb * p.mod.bsb + (int64_t)hh * p.mod.bsh +
-                                            (int64_t)q_row * p.mod.bsq + (int64_t)j * kTileRows
-                                      : nullptr,
-                                1, 1.f / p.scale);
+      if (dense || (alibi && !alibi_inline)) {
+        bias_scores_tmem<true>(tmem_S[t] + lane_off, kTileRows, alibi && !alibi_inline, alibi_over_scale, qpos,
+                               p.mod.kv_pos + kv0,
+                               dense ? p.mod.bias + (int64_t)bb * p.mod.bsb + (int64_t)hh * p.mod.bsh +
+                                           (int64_t)q_row * p.mod.bsq + (int64_t)j * kTileRows
+                                     : nullptr,
+                               1, 1.f / p.scale);
       }
       uint32_t r[4][32];
 #pragma unroll
@@ -293,6 +311,13 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
             r[c][e] = __float_as_uint(fmaf(slope2, (float)(c * 32 + e), fmaf(__uint_as_float(r[c][e]), scale2, r_i)));
         sc = 1.f;
       }
+      if (need_mask) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+          for (int e = 0; e < 32; ++e)
+            if (!((vis[c] >> e) & 1u)) r[c][e] = 0xff800000u;  // -inf
+      }
       // raw scores; the scale is positive, so it commutes with max.  Four independent chains of
       // three-input maxima instead of one chain of 128 dependent operations.
       float mxa[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -309,7 +334,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
         m_ref = m_new;
         l_run *= alpha;
         alpha_total *= alpha;
-        if (i > 0) {  // O of this tile holds the sum over the tiles before this one
+        if (done > 0) {  // O of this tile holds the sum over the tiles before this one
 #pragma unroll 1
           for (int c = 0; c < D / 16; ++c) {
             uint32_t o[16];
@@ -355,6 +380,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
       tc_wait_st();
       tc_fence_before();
       mbar_arrive(&bars[P_FULL0 + t]);
+      ++done;
     }
 
     // Epilogue: fold in the carried state of earlier ring steps, bring (o, m, l) to the
@@ -374,7 +400,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
 #pragma unroll 1
       for (int c = 0; c < D / 8; ++c) {
         uint32_t o[8];
-        if (count > 0) {
+        if (done > 0) {
           tmem_ld8(tmem_O[t] + lane_off + c * 8, o);
           tc_wait_ld();
         } else {
@@ -496,7 +522,7 @@ EncodeTiledFn encode_fn() {
 
 template <int D>
 cudaError_t launch_fwd(const FwdTcParams& P, cudaStream_t s) {
-  constexpr size_t kSmem = 6 * kTileRows * D * 2 + kMaxTiles * 3 + NUM_BARS * 8 + 64 + 1024;
+  constexpr size_t kSmem = 6 * kTileRows * D * 2 + kMaxTiles * 5 + NUM_BARS * 8 + 64 + 1024;
   constexpr size_t kRequest = kSmem < 120 * 1024 ? 120 * 1024 : kSmem;  // one CTA per SM: it owns all of TMEM
   auto kern = tc_fwd_kernel<D>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRequest);
