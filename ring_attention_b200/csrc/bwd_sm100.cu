@@ -27,6 +27,12 @@
 // memory delivers, so every other access on that data path (TMA writes of Q and dO, the dS^T
 // stores, the loads of the per-row terms, global reductions) lengthens the MMAs.  That is why
 // dQ leaves through registers and not through a shared-memory staging buffer as well.
+// RAGGED: query or key rows that are not a multiple of 128, results in bf16.  TMA fills the rows past
+// the tensors with zeros; pairs past either end are masked, rows past them are not stored or added.
+// These calls used to run on the CUDA cores with P and dS in fp32, so both keep 16 bits here: two bf16
+// halves each (P^T hi and lo in the two halves of a warpgroup's S^T columns, dS^T in two shared-memory
+// tiles), and dV, dK and dQ take two MMAs per k-step.  At head dim 128 the second dS^T tile takes the
+// room of the second dO stage.
 // Head dim 128: warps 0-7 compute (two warpgroups split the 128 query columns), warps 8-11 drain
 // dQ^T, warp 12 TMA producer, warp 13 MMA issuer, warps 14-15 idle (registers are re-divided
 // between whole warpgroups).  Head dim 64: warps 0-7 compute, warp 8 producer, warp 9 MMA issuer.
@@ -59,6 +65,8 @@ __device__ __forceinline__ void reg_dec() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
+__host__ __device__ constexpr int bwd_do_stages(int d, bool ragged) { return ragged && d == 128 ? 1 : 2; }
+
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr unsigned kProducerPollNs = 100;
 
@@ -89,7 +97,7 @@ __device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float 
                : "memory");
 }
 
-template <int D>
+template <int D, bool RAGGED>
 __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const __grid_constant__ BwdTcParams P) {
   constexpr bool DRAIN = D == 128;  // the drain warpgroup serves the dQ^T form
   constexpr int PRODUCER_WARP = DRAIN ? 12 : 8, MMA_WARP = PRODUCER_WARP + 1;
@@ -97,14 +105,15 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
   constexpr int PANELS = D / 64;
   constexpr int PANEL_BYTES = kTileRows * 128;
   constexpr int DS_BYTES = kTileRows * kTileRows * 2;
-  constexpr int DO_ST = 2;
+  constexpr int DO_ST = bwd_do_stages(D, RAGGED);
+  constexpr int DS_TILES = RAGGED ? 2 : 1;  // dS^T, and what its rounding to bf16 left
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sK = smem;
   uint8_t* sV = sK + TILE_BYTES;
   uint8_t* sQ = sV + TILE_BYTES;          // 2 stages
   uint8_t* sdO = sQ + 2 * TILE_BYTES;     // DO_ST stages
   uint8_t* sdS = sdO + DO_ST * TILE_BYTES;  // [128 key rows][128 query cols] bf16, 2 panels, 128B swizzle
-  float* sL = reinterpret_cast<float*>(sdS + DS_BYTES);  // [2][128]
+  float* sL = reinterpret_cast<float*>(sdS + DS_TILES * DS_BYTES);  // [2][128]
   float* sDelta = sL + 2 * kTileRows;                     // [2][128]
   uint64_t* bars = reinterpret_cast<uint64_t*>(sDelta + 2 * kTileRows);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NUM_BARS);
@@ -123,7 +132,7 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
   const int hh = bh % p.h, bb = bh / p.h;
   const uint32_t kinds = p.mod.kinds;
   const bool masked = (kinds & kMetaKinds) != 0;  // the tile summaries are read
-  const bool dense = (kinds & RA_MOD_DENSE) != 0;  // every tile takes the in-TMEM pass that adds the bias tile
+  const bool dense = !RAGGED && (kinds & RA_MOD_DENSE) != 0;  // every tile takes the in-TMEM pass that adds the bias tile
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < NUM_BARS; ++i) {
@@ -220,7 +229,7 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
     // Two streams of loads: Q (with L and delta of its rows) and dO.  A Q stage is free after
     // dK of its tile, a dO stage already after dV of its tile, one MMA group earlier in the
     // next iteration: dO runs further ahead.  Both are polled so that neither blocks the other.
-    const int64_t row_base = ((int64_t)bb * p.h + hh) * p.lq;
+    const int64_t row_base = ((int64_t)bb * p.h + hh) * P.n_q_tiles * kTileRows;  // the row terms are padded to whole tiles
     int qi = i, doi = i, qn = 0, don = 0;
     long long t0 = 0;
     uint32_t idle = 0;
@@ -286,6 +295,7 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
       // Low descriptor words: K-major views step 32 B per k-step inside a 64-column panel and one
       // panel (16 KB) per 4 k-steps; MN-major views step 16 rows (2 KB) per k-step, panels 16 KB apart.
       constexpr uint32_t kPanel16 = PANEL_BYTES >> 4, kStage16 = TILE_BYTES >> 4;
+      constexpr uint32_t kLow16 = DS_BYTES >> 4;  // from a dS^T tile to its low half
       const uint32_t k_km = desc_lo(smem_u32(sK), 16), k_mn = desc_lo(smem_u32(sK), PANEL_BYTES);
       const uint32_t v_km = desc_lo(smem_u32(sV), 16);
       const uint32_t q_km = desc_lo(smem_u32(sQ), 16), q_mn = desc_lo(smem_u32(sQ), PANEL_BYTES);
@@ -313,6 +323,11 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
         for (int kk = 0; kk < 8; ++kk) {
           const uint32_t pcol = kk < 4 ? kk * 8 : 64 + (kk - 4) * 8;  // P^T columns of the two warpgroups
           mma_ts_warp(tmem_dV, tmem_S + pcol, desc_from_lo(b0 + mn_off(kk)), idesc_dv, (!first_tile) || kk > 0);
+        }
+        if constexpr (RAGGED) {  // the low halves: 32 columns behind the high ones
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)
+            mma_ts_warp(tmem_dV, tmem_S + (kk < 4 ? kk * 8 : 64 + (kk - 4) * 8) + 32, desc_from_lo(b0 + mn_off(kk)), idesc_dv, 1u);
         }
       };
       // Issue order per query tile n (the tensor pipe executes in this order):
@@ -358,10 +373,20 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk)
               mma_ss_warp(tmem_dP, desc_from_lo(k_mn + mn_off(kk)), desc_from_lo(ds_mn + mn_off(kk)), idesc_dq, kk > 0);
+            if constexpr (RAGGED) {
+#pragma unroll
+              for (int kk = 0; kk < 8; ++kk)
+                mma_ss_warp(tmem_dP, desc_from_lo(k_mn + mn_off(kk)), desc_from_lo(ds_mn + kLow16 + mn_off(kk)), idesc_dq, 1u);
+            }
           } else {
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk)
               mma_ss_warp(tmem_dP, desc_from_lo(ds_mn + mn_off(kk)), desc_from_lo(k_mn + mn_off(kk)), idesc_dq, kk > 0);
+            if constexpr (RAGGED) {
+#pragma unroll
+              for (int kk = 0; kk < 8; ++kk)
+                mma_ss_warp(tmem_dP, desc_from_lo(ds_mn + kLow16 + mn_off(kk)), desc_from_lo(k_mn + mn_off(kk)), idesc_dq, 1u);
+            }
           }
           tc_commit_warp(&bars[DQ_FULL]);
           {
@@ -370,6 +395,11 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
             for (int kk = 0; kk < 8; ++kk)
               mma_ss_warp(tmem_dK, desc_from_lo(ds_km + km_off(kk)), desc_from_lo(b0 + mn_off(kk)), idesc_dv,
                      (n > 0) || kk > 0);
+            if constexpr (RAGGED) {
+#pragma unroll
+              for (int kk = 0; kk < 8; ++kk)
+                mma_ss_warp(tmem_dK, desc_from_lo(ds_km + kLow16 + km_off(kk)), desc_from_lo(b0 + mn_off(kk)), idesc_dv, 1u);
+            }
           }
           tc_commit_warp(&bars[Q_EMPTY0 + s]);
           if (!has_next) break;
@@ -409,10 +439,12 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
         tc_wait_ld();
         tc_fence_before();
         mbar_arrive(&bars[DQ_DRAINED]);
+        const int q_left = p.lq - i * kTileRows;  // a ragged last tile: rows past lq are another head's
         float* base = p.dq + (qrow_base + (int64_t)i * kTileRows) * 128 + r;
 #pragma unroll
         for (int c = 0; c < 128; ++c)
-          asm volatile("red.global.add.f32 [%0], %1;" ::"l"(base + c * 128), "f"(__uint_as_float(dv[c >> 5][c & 31])) : "memory");
+          if (!RAGGED || c < q_left)
+            asm volatile("red.global.add.f32 [%0], %1;" ::"l"(base + c * 128), "f"(__uint_as_float(dv[c >> 5][c & 31])) : "memory");
         i = next_active(win, i + 1) & kTileIdx;
       }
     }
@@ -427,9 +459,11 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
     const bool alibi = (kinds & RA_MOD_ALIBI) != 0;
     int32_t kpos = 0, kseg = 0;
     bool kpre = false;
-    if (p.mod.kv_pos) kpos = p.mod.kv_pos[(int64_t)bb * p.lk + kv_row];
-    if (p.mod.kv_seg) kseg = p.mod.kv_seg[(int64_t)bb * p.lk + kv_row];
-    if (p.mod.kv_pre) kpre = p.mod.kv_pre[(int64_t)bb * p.lk + kv_row] != 0;
+    const bool row_valid = !RAGGED || kv_row < p.lk;
+    const int64_t mod_row = (int64_t)bb * p.lk + (row_valid ? kv_row : p.lk - 1);
+    if (p.mod.kv_pos) kpos = p.mod.kv_pos[mod_row];
+    if (p.mod.kv_seg) kseg = p.mod.kv_seg[mod_row];
+    if (p.mod.kv_pre) kpre = p.mod.kv_pre[mod_row] != 0;
     const int64_t qrow_base = ((int64_t)bb * p.h + hh) * p.lq;
     bool ok = true;  // warp-uniform: the tile scan below votes across the warp
     float pf[64];        // P^T of the tile whose dS^T is formed next (this thread's row, 64 columns)
@@ -465,16 +499,20 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
         auto ds_chunk = [&](int ch, const uint32_t* dp) {
           const float4 da = Dls[ch * 2], db = Dls[ch * 2 + 1];  // -delta * scale of 8 queries
           const uint64_t dl2[4] = {pack2(da.x, da.y), pack2(da.z, da.w), pack2(db.x, db.y), pack2(db.z, db.w)};
-          uint32_t w[4];
+          uint32_t w[4], wl[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const int c = ch * 8 + e * 2;
             const uint64_t dp2 = pack2(__uint_as_float(dp[e * 2]), __uint_as_float(dp[e * 2 + 1]));
             float d0, d1;
             unpack2(mul2(pack2(pf[c], pf[c + 1]), fma2(dp2, scl2, dl2[e])), d0, d1);
+            if (RAGGED && !row_valid) d0 = d1 = 0.f;  // P is 0 there, but dP may not be finite
             w[e] = pack_bf16(d0, d1);
+            if constexpr (RAGGED) wl[e] = pack_bf16_rest(w[e], d0, d1);
           }
           *reinterpret_cast<uint4*>(row_ptr + ((ch ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+          if constexpr (RAGGED)
+            *reinterpret_cast<uint4*>(row_ptr + DS_BYTES + ((ch ^ (r & 7)) << 4)) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
         };
         if constexpr (DRAIN) {
           // fewer registers per thread here: the second 32 columns are loaded once half of the
@@ -498,15 +536,19 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
       if (have_cur) {
         // ---- P^T = exp2(S^T * scale2 - L * log2e) of tile k on this warpgroup's 64 query columns
         const int n = k, s = n & 1, i = i_cur;
-        const bool need_mask = (e_cur & kMixedBit) != 0;
+        const int ncols = (RAGGED ? min(kTileRows, p.lq - i * kTileRows) : kTileRows) - g * 64;  // query rows this warpgroup has
+        // at either ragged end the pairs past it are masked
+        const bool need_mask = (e_cur & kMixedBit) != 0 || (RAGGED && (ncols < 64 || (kt + 1) * kTileRows > p.lk));
         // ALiBi over a tile of contiguous query positions is two FMAs per score in registers, over
         // scattered ones it takes the in-TMEM pass below
         const bool alibi_inline = alibi && (e_cur & kContigBit) != 0;
         const int64_t q0 = (int64_t)bb * p.lq + (int64_t)i * kTileRows + g * 64;
         uint32_t vis[2];
-        if (need_mask)  // found while the scores are on their way
+        if (need_mask) {  // found while the scores are on their way
           visible_columns<false>(vis, kinds, p.mod.window, kpos, kseg, kpre, p.mod.q_pos + q0, p.mod.q_seg + q0,
-                                 p.mod.q_pre + q0, q0_cur + g * 64, (e_cur & kContigBit) != 0);
+                                 p.mod.q_pre + q0, q0_cur + g * 64, (e_cur & kContigBit) != 0, RAGGED ? ncols : 64);
+          if (RAGGED && !row_valid) vis[0] = vis[1] = 0u;
+        }
         if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[Q_FULL0 + s], (n >> 1) & 1, abort_flag, P.status, kStBwdCompute)))) break;
         const float4* Ls = reinterpret_cast<const float4*>(sL + s * kTileRows + g * 64);
         if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[S_FULL], n & 1, abort_flag, P.status, kStBwdCompute)))) break;
@@ -517,7 +559,7 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
                                   dense ? p.mod.bias + (int64_t)bb * p.mod.bsb + (int64_t)hh * p.mod.bsh +
                                               ((int64_t)i * kTileRows + g * 64) * p.mod.bsq + kv_row
                                         : nullptr,
-                                  p.mod.bsq, 1.f / p.scale);
+                                  p.mod.bsq, 1.f / p.scale, RAGGED ? ncols : 64);
         }
         tmem_ld32(tmem_S + lane_off + g * 64, sv[0]);
         tmem_ld32(tmem_S + lane_off + g * 64 + 32, sv[1]);
@@ -577,6 +619,11 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
 #pragma unroll
           for (int e = 0; e < 16; ++e) pk[e] = pack_bf16(pf[32 * hf + 2 * e], pf[32 * hf + 2 * e + 1]);
           tmem_st16(tmem_S + lane_off + g * 64 + 16 * hf, pk);
+          if constexpr (RAGGED) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) pk[e] = pack_bf16_rest(pk[e], pf[32 * hf + 2 * e], pf[32 * hf + 2 * e + 1]);
+            tmem_st16(tmem_S + lane_off + g * 64 + 32 + 16 * hf, pk);
+          }
         }
         tc_wait_st();
         tc_fence_before();
@@ -592,9 +639,10 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
           float* dq_row = p.dq + (qrow_base + (int64_t)i_prev * kTileRows + r) * D + g * HALF;
           tmem_ld32(tmem_dP + lane_off + g * HALF, sv[0]);
           tc_wait_ld();
+          const bool q_valid = !RAGGED || i_prev * kTileRows + r < p.lq;
 #pragma unroll
           for (int e = 0; e < 32; e += 4)
-            red_add_v4(dq_row + e, __uint_as_float(sv[0][e]), __uint_as_float(sv[0][e + 1]), __uint_as_float(sv[0][e + 2]),
+            if (q_valid) red_add_v4(dq_row + e, __uint_as_float(sv[0][e]), __uint_as_float(sv[0][e + 1]), __uint_as_float(sv[0][e + 2]),
                        __uint_as_float(sv[0][e + 3]));
           tc_fence_before();
           mbar_arrive(&bars[DQ_DRAINED]);
@@ -615,7 +663,7 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
       const int64_t krow = ((int64_t)bb * p.h + hh) * p.lk + kv_row;
       float* dk_row = p.dk + krow * D + g * HALF;
       float* dv_row = p.dv + krow * D + g * HALF;
-      const bool direct = p.dk_out.ptr != nullptr;  // ring of one: results go out in the input dtype
+      const bool direct = RAGGED || p.dk_out.ptr != nullptr;  // ring of one: results go out in the input dtype
       const bool fresh = p.overwrite != 0;          // the fp32 buffers hold nothing yet: store, do not add
       __nv_bfloat16* dk_o = direct ? (__nv_bfloat16*)p.dk_out.ptr + (int64_t)bb * p.dk_out.sb +
                                          (int64_t)kv_row * p.dk_out.sl + (int64_t)hh * p.dk_out.sh + g * HALF
@@ -634,7 +682,7 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
           w.y = pack_bf16(__uint_as_float(a[2]), __uint_as_float(a[3]));
           w.z = pack_bf16(__uint_as_float(a[4]), __uint_as_float(a[5]));
           w.w = pack_bf16(__uint_as_float(a[6]), __uint_as_float(a[7]));
-          *reinterpret_cast<uint4*>(dk_o + c * 8) = w;
+          if (row_valid) *reinterpret_cast<uint4*>(dk_o + c * 8) = w;
         } else {
 #pragma unroll
           for (int e = 0; e < 8; e += 4) {
@@ -654,7 +702,7 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
           w.y = pack_bf16(__uint_as_float(a[2]), __uint_as_float(a[3]));
           w.z = pack_bf16(__uint_as_float(a[4]), __uint_as_float(a[5]));
           w.w = pack_bf16(__uint_as_float(a[6]), __uint_as_float(a[7]));
-          *reinterpret_cast<uint4*>(dv_o + c * 8) = w;
+          if (row_valid) *reinterpret_cast<uint4*>(dv_o + c * 8) = w;
         } else {
 #pragma unroll
           for (int e = 0; e < 8; e += 4) {
@@ -667,7 +715,7 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
           }
         }
       }
-    } else if (ok && n == 0 && p.dk_out.ptr != nullptr) {
+    } else if (ok && n == 0 && p.dk_out.ptr != nullptr && row_valid) {
       // no query tile sees this K/V tile: its gradients are zero, and in direct mode nobody else writes them
       constexpr int HALF = D / 2;
       __nv_bfloat16* dk_o = (__nv_bfloat16*)p.dk_out.ptr + (int64_t)bb * p.dk_out.sb + (int64_t)kv_row * p.dk_out.sl +
@@ -680,7 +728,7 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
         *reinterpret_cast<uint4*>(dv_o + c * 8) = make_uint4(0u, 0u, 0u, 0u);
       }
     }
-    else if (ok && n == 0 && p.overwrite) {
+    else if (ok && n == 0 && p.overwrite && !RAGGED) {
       // no query tile sees this K/V tile and the fp32 buffers were not cleared: its rows are zero
       constexpr int HALF = D / 2;
       const int64_t krow = ((int64_t)bb * p.h + hh) * p.lk + kv_row;
@@ -700,11 +748,11 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
   }
 }
 
-template <int D>
+template <int D, bool RAGGED>
 cudaError_t launch_bwd(const BwdTcParams& P, cudaStream_t s) {
-  constexpr size_t kSmem = 6 * kTileRows * D * 2 + kTileRows * kTileRows * 2 + 4 * kTileRows * 4 + NUM_BARS * 8 + 64;
+  constexpr size_t kSmem = (4 + bwd_do_stages(D, RAGGED)) * kTileRows * D * 2 + (RAGGED ? 2 : 1) * kTileRows * kTileRows * 2 + 4 * kTileRows * 4 + NUM_BARS * 8 + 64;
   constexpr size_t kRequest = kSmem < 120 * 1024 ? 120 * 1024 : kSmem;  // one CTA per SM: it owns all of TMEM
-  auto kern = tc_bwd_kernel<D>;
+  auto kern = tc_bwd_kernel<D, RAGGED>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRequest);
   if (e != cudaSuccess) return e;
   kern<<<P.n_kv_tiles * P.p.b * P.p.h, bwd_threads(D == 128), kRequest, s>>>(P);
@@ -718,11 +766,10 @@ bool aligned16(const TensorView& t) {
 
 }  // namespace
 
-const char* tc_bwd_unsupported_reason(const BwdParams& p, int dtype) {
+static const char* bwd_unsupported_reason(const BwdParams& p, int dtype) {
   if (dtype != RA_DTYPE_BF16) return "inputs are not bf16";
   if (p.dk_dim != p.dv_dim || (p.dk_dim != 64 && p.dk_dim != 128)) return "head dims must be equal and 64 or 128";
-  if (p.lq % kTileRows || p.lk % kTileRows) return "lq and lk must be multiples of 128";
-  if (p.lq / kTileRows > kMaxTiles || p.lk / kTileRows > kMaxTiles) return "more than 4096 tiles along one axis";
+  if (tiles_of(p.lq) > kMaxTiles || tiles_of(p.lk) > kMaxTiles) return "more than 4096 tiles along one axis";
   if ((p.mod.kinds & RA_MOD_DENSE) && ((p.mod.bsb % 4) || (p.mod.bsh % 4) || (p.mod.bsq % 4) ||
                                        (reinterpret_cast<uintptr_t>(p.mod.bias) & 15)))
     return "the dense bias needs a 16-byte aligned base and strides that are multiples of 4 floats";
@@ -738,12 +785,24 @@ const char* tc_bwd_unsupported_reason(const BwdParams& p, int dtype) {
   return nullptr;
 }
 
+const char* tc_bwd_unsupported_reason(const BwdParams& p, int dtype) {
+  if (p.lq % kTileRows || p.lk % kTileRows) return "lq and lk must be multiples of 128";
+  return bwd_unsupported_reason(p, dtype);
+}
+
+const char* tc_bwd_ragged_unsupported_reason(const BwdParams& p, int dtype) {
+  if (!(p.lq % kTileRows || p.lk % kTileRows)) return "lq and lk are multiples of 128";
+  if (!p.dk_out.ptr) return "ragged lengths are served for whole attentions with bf16 results";
+  if (p.mod.kinds & RA_MOD_DENSE) return "ragged lengths are not served with a dense bias tile";
+  return bwd_unsupported_reason(p, dtype);
+}
+
 cudaError_t tc_bwd_block(const BwdParams& p, cudaStream_t s) {
   BwdTcParams P;
   memset(&P, 0, sizeof(P));
   P.p = p;
-  P.n_q_tiles = p.lq / kTileRows;
-  P.n_kv_tiles = p.lk / kTileRows;
+  P.n_q_tiles = tiles_of(p.lq);
+  P.n_kv_tiles = tiles_of(p.lk);
   const char* why = nullptr;
   if (!make_tile_map(&P.map_q, p.q, p.b, p.lq, p.h, p.dk_dim, kTileRows, &why) ||
       !make_tile_map(&P.map_k, p.k, p.b, p.lk, p.h, p.dk_dim, kTileRows, &why) ||
@@ -763,12 +822,13 @@ cudaError_t tc_bwd_block(const BwdParams& p, cudaStream_t s) {
   float* terms = nullptr;
   cudaError_t e = cudaSuccess;
   if (!p.row_nl2 || !p.row_nds) {  // block-level callers pass L and delta as the reference does
-    const int64_t rows = (int64_t)p.b * p.h * p.lq;
+    const int64_t rows = (int64_t)p.b * p.h * P.n_q_tiles * kTileRows;
     const size_t each = ((size_t)rows * sizeof(float) + 255) / 256 * 256;
     if ((e = scratch_alloc((void**)&terms, 2 * each, s)) != cudaSuccess) return e;
     float* nl2 = terms;
     float* nds = reinterpret_cast<float*>(reinterpret_cast<char*>(terms) + each);
-    e = launch_bwd_row_terms(p.lse, p.delta, p.scale, (p.mod.kinds & RA_MOD_DENSE) ? 0 : 1, rows, nl2, nds, s);
+    e = launch_bwd_row_terms(p.lse, p.delta, p.scale, (p.mod.kinds & RA_MOD_DENSE) ? 0 : 1, (int64_t)p.b * p.h, p.lq,
+                             P.n_q_tiles * kTileRows, nl2, nds, s);
     P.p.row_nl2 = nl2;
     P.p.row_nds = nds;
   }
@@ -785,7 +845,11 @@ cudaError_t tc_bwd_block(const BwdParams& p, cudaStream_t s) {
     P.meta_q = mq;
     P.meta_kv = mk;
   }
-  if (e == cudaSuccess) e = p.dk_dim == 128 ? launch_bwd<128>(P, s) : launch_bwd<64>(P, s);
+  const bool ragged = p.lq % kTileRows || p.lk % kTileRows;
+  if (e == cudaSuccess) {
+    if (ragged) e = p.dk_dim == 128 ? launch_bwd<128, true>(P, s) : launch_bwd<64, true>(P, s);
+    else e = p.dk_dim == 128 ? launch_bwd<128, false>(P, s) : launch_bwd<64, false>(P, s);
+  }
   if (meta) cudaFreeAsync(meta, s);  // stream-ordered: after the kernels above, also when one failed to launch
   if (terms) cudaFreeAsync(terms, s);
   return e;

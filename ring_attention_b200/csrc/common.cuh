@@ -53,6 +53,7 @@ struct BwdParams {
   // its inner loops, computed once per backward instead of once per tile and thread:
   //   row_nl2 = min(-lse * log2(e), 1e30)  (no clamp with a dense bias tile: ring.py:146 as it is)
   //   row_nds = -delta * scale
+  // with lq padded to a multiple of 128 per (batch, head).
   // When they are NULL the launcher derives them into scratch first.
   const float* row_nl2;
   const float* row_nds;
@@ -83,9 +84,10 @@ cudaError_t launch_delta(int b, int h, int lq, int dv, TensorView out, TensorVie
                          float* delta, cudaStream_t s);
 cudaError_t launch_cast_from_f32(int b, int h, int len, int d, const float* src, TensorView dst,
                                  int dtype, cudaStream_t s);
-// nl2[i] = min(-lse[i] * log2(e), 1e30) (clamp left out when !clamp), nds[i] = -delta[i] * scale.
-cudaError_t launch_bwd_row_terms(const float* lse, const float* delta, float scale, int clamp, int64_t n, float* nl2,
-                                 float* nds, cudaStream_t s);
+// nl2 = min(-lse * log2(e), 1e30) (clamp left out when !clamp), nds = -delta * scale, for bh runs of lq rows;
+// the results have `pitch` >= lq rows per run, of which the last pitch - lq are padding.
+cudaError_t launch_bwd_row_terms(const float* lse, const float* delta, float scale, int clamp, int64_t bh, int lq,
+                                 int pitch, float* nl2, float* nds, cudaStream_t s);
 cudaError_t launch_add_f32(float* dst, const float* src, int64_t n, cudaStream_t s);
 // dst[seg * pitch + i] += src[seg * pitch + i] for seg < nseg, i < seg_elems (a multiple of 4; 16-byte aligned rows).
 cudaError_t launch_add_rows_f32(float* dst, const float* src, int64_t nseg, int64_t seg_elems, int64_t pitch, cudaStream_t s);

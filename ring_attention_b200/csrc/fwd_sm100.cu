@@ -14,6 +14,11 @@
 // K/V layout, so nothing is transposed.  Running max / sum live in registers; O in TMEM
 // is rescaled only when the row max grows by more than 2^8, and the carried O of earlier
 // ring steps is folded in once, in the epilogue.
+// RAGGED: query or key rows that are not a multiple of 128, results in bf16.  The last tiles run past
+// the tensors: TMA fills their rows with zeros, the columns past lk are masked, rows past lq are not
+// stored.  These calls used to run on the CUDA cores with P in fp32, so here P keeps 16 bits: it goes
+// to TMEM as two bf16 halves (hi in the first, lo in the second half of S's columns) and PV runs twice;
+// every exponential is ex2.  What bounds it is the same softmax path plus 1.5 times the MMAs.
 // TMEM columns: S0 [0,128) S1 [128,256) O0 [256,256+D) O1 [256+D,256+2D).
 #include <cstdio>
 #include <cstring>
@@ -58,7 +63,7 @@ enum Bar {
   S_FULL0, S_FULL1, P_FULL0, P_FULL1, O_FULL, NUM_BARS
 };
 
-template <int D>
+template <int D, bool RAGGED>
 __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_constant__ FwdTcParams P) {
   constexpr int TILE_BYTES = kTileRows * D * 2;
   constexpr int PANELS = D / 64;           // 64-element (128-byte) panels per row
@@ -104,7 +109,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
   // Every thread classifies its share of the tiles (one round of loads for up to 320 tiles), then
   // warp 0 compacts the classes in order.
   const bool masked = (kinds & kMetaKinds) != 0;
-  const bool dense = (kinds & RA_MOD_DENSE) != 0;
+  const bool dense = !RAGGED && (kinds & RA_MOD_DENSE) != 0;
   const uint32_t all_visible = ntile == 2 ? (kVisible << 0) | (kVisible << 1) : kVisible;
   if (masked) {
     const TileMeta mq0 = P.meta_q[bb * P.n_q_tiles + qt0];
@@ -129,6 +134,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
         code = (uint32_t)codes[j] << kTileBits;
         active = (code & all_visible) != 0;
       }
+      // the last tile's columns past lk are masked (kMixed is kVisible << 2)
+      if (RAGGED && j == P.n_kv_tiles - 1 && p.lk % kTileRows) code |= (code & all_visible) << 2;
       const uint32_t vote = __ballot_sync(0xffffffffu, active);
       if (active) list[cnt + __popc(vote & ((1u << lane) - 1))] = (uint32_t)j | code;
       cnt += __popc(vote);
@@ -206,6 +213,11 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
         for (int kk = 0; kk < kTileRows / 16; ++kk)
           mma_ts_warp(tmem_O[t], tmem_S[t] + kk * 8, desc_from_lo(b0 + kk * (2048 >> 4)), idesc_pv,
                  (!first_tile) || kk > 0);
+        if constexpr (RAGGED) {  // the low half of P
+#pragma unroll
+          for (int kk = 0; kk < kTileRows / 16; ++kk)
+            mma_ts_warp(tmem_O[t], tmem_S[t] + 64 + kk * 8, desc_from_lo(b0 + kk * (2048 >> 4)), idesc_pv, 1u);
+        }
       };
       for (int t = 0; t < ntile && ok; ++t)
         ok = __all_sync(0xffffffffu, mbar_wait(&bars[Q_FULL0 + t], 0, abort_flag, P.status, kStFwdMma));
@@ -249,16 +261,18 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
     const float scale2 = p.scale * kLog2e;
 
     float m_ref = -INFINITY, l_run = 0.f, alpha_total = 1.f;
-    if (!p.first) {
+    if (!RAGGED && !p.first) {
       m_ref = p.m[state_row] * kLog2e;
       l_run = p.l[state_row];
     }
     float m_true = m_ref;
     int32_t qpos = 0, qseg = 0;
     bool qpre = false;
-    if (p.mod.q_pos) qpos = p.mod.q_pos[(int64_t)bb * p.lq + q_row];
-    if (p.mod.q_seg) qseg = p.mod.q_seg[(int64_t)bb * p.lq + q_row];
-    if (p.mod.q_pre) qpre = p.mod.q_pre[(int64_t)bb * p.lq + q_row] != 0;
+    const bool row_valid = !RAGGED || q_row < p.lq;
+    const int64_t mod_row = (int64_t)bb * p.lq + (row_valid ? q_row : p.lq - 1);
+    if (p.mod.q_pos) qpos = p.mod.q_pos[mod_row];
+    if (p.mod.q_seg) qseg = p.mod.q_seg[mod_row];
+    if (p.mod.q_pre) qpre = p.mod.q_pre[mod_row] != 0;
     const bool alibi = (kinds & RA_MOD_ALIBI) != 0;
     bool ok = true;
 
@@ -280,10 +294,11 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
       if (has_pos && i + 1 < count) k0_next = p.mod.kv_pos[(int64_t)bb * p.lk + (int64_t)(list[i + 1] & kTileIdx) * kTileRows];
       if (!(entry & (kVisible << t))) continue;
       const int64_t kv0 = (int64_t)bb * p.lk + (int64_t)j * kTileRows;
+      const int ncols = RAGGED ? min(kTileRows, p.lk - j * kTileRows) : kTileRows;  // key rows of this tile
       uint32_t vis[4];
       if (need_mask)  // a tile that mixes visible and masked pairs: found while its scores are on their way
         visible_columns<true>(vis, kinds, p.mod.window, qpos, qseg, qpre, p.mod.kv_pos + kv0, p.mod.kv_seg + kv0,
-                              p.mod.kv_pre + kv0, k0, kv_contig);
+                              p.mod.kv_pre + kv0, k0, kv_contig, ncols);
       if (!(ok = mbar_wait(&bars[S_FULL0 + t], done & 1, abort_flag, P.status, kStFwdSoftmax))) break;
       tc_fence_after();
       if (dense || (alibi && !alibi_inline)) {
@@ -292,7 +307,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
                                dense ? p.mod.bias + (int64_t)bb * p.mod.bsb + (int64_t)hh * p.mod.bsh +
                                            (int64_t)q_row * p.mod.bsq + (int64_t)j * kTileRows
                                      : nullptr,
-                               1, 1.f / p.scale);
+                               1, 1.f / p.scale, ncols);
       }
       uint32_t r[4][32];
 #pragma unroll
@@ -354,12 +369,12 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
       uint64_t sum2[4] = {0ull, 0ull, 0ull, 0ull};
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        uint32_t pk[16];
+        uint32_t pk[16], pl[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
           const uint64_t x2 = fma2(pack2(__uint_as_float(r[c][2 * e]), __uint_as_float(r[c][2 * e + 1])), sc2, nm2);
           float p0, p1;
-          if (e < kPolyPairs) {
+          if (!RAGGED && e < kPolyPairs) {
             exp2_poly2(x2, p0, p1);
           } else {
             float x0, x1;
@@ -369,8 +384,10 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
           }
           sum2[c] = add2(sum2[c], pack2(p0, p1));
           pk[e] = pack_bf16(p0, p1);
+          if constexpr (RAGGED) pl[e] = pack_bf16_rest(pk[e], p0, p1);
         }
         tmem_st16(tmem_S[t] + lane_off + c * 16, pk);
+        if constexpr (RAGGED) tmem_st16(tmem_S[t] + lane_off + 64 + c * 16, pl);
       }
       {
         float s0, s1;
@@ -389,9 +406,10 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
     if (ok) {
       tc_fence_after();
       const float beta = (m_ref == -INFINITY) ? 1.f : ex2(m_ref - m_true);
-      const float in_scale = p.first ? 0.f : alpha_total * beta;
+      const bool first = RAGGED || p.first;  // a ragged call is the whole attention: no carried state, results go out
+      const float in_scale = first ? 0.f : alpha_total * beta;
       float* o_row = p.o + state_row * D;
-      const bool finalize = p.final_out.ptr != nullptr;
+      const bool finalize = RAGGED || p.final_out.ptr != nullptr;
       const float l_tot = l_run * beta;
       const float inv_l = 1.f / l_tot;  // l = 0 (a row that saw no key) gives 0 * inf = NaN, as o / l does
       __nv_bfloat16* out_row = finalize ? (__nv_bfloat16*)p.final_out.ptr + (int64_t)bb * p.final_out.sb +
@@ -411,7 +429,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
 #pragma unroll
         for (int e = 0; e < 8; e += 4) {
           float4 prev = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (!p.first) prev = *reinterpret_cast<const float4*>(o_row + c * 8 + e);
+          if (!first) prev = *reinterpret_cast<const float4*>(o_row + c * 8 + e);
           val[e] = __uint_as_float(o[e]) * beta + prev.x * in_scale;
           val[e + 1] = __uint_as_float(o[e + 1]) * beta + prev.y * in_scale;
           val[e + 2] = __uint_as_float(o[e + 2]) * beta + prev.z * in_scale;
@@ -423,14 +441,14 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
           w.y = pack_bf16(val[2] * inv_l, val[3] * inv_l);
           w.z = pack_bf16(val[4] * inv_l, val[5] * inv_l);
           w.w = pack_bf16(val[6] * inv_l, val[7] * inv_l);
-          *reinterpret_cast<uint4*>(out_row + c * 8) = w;
+          if (row_valid) *reinterpret_cast<uint4*>(out_row + c * 8) = w;
         } else {
           *reinterpret_cast<float4*>(o_row + c * 8) = make_float4(val[0], val[1], val[2], val[3]);
           *reinterpret_cast<float4*>(o_row + c * 8 + 4) = make_float4(val[4], val[5], val[6], val[7]);
         }
       }
       if (finalize) {
-        if (p.final_lse) p.final_lse[state_row] = m_true * (1.f / kLog2e) + logf(l_tot);
+        if (p.final_lse && row_valid) p.final_lse[state_row] = m_true * (1.f / kLog2e) + logf(l_tot);
       } else {
         p.m[state_row] = m_true * (1.f / kLog2e);
         p.l[state_row] = l_tot;
@@ -450,15 +468,16 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
 // -----------------------------------------------------------------------------------------
 __global__ void tile_meta_kernel(TileMeta* __restrict__ out, const int32_t* __restrict__ pos,
                                  const int32_t* __restrict__ seg, const uint8_t* __restrict__ pre, int len) {
-  // one warp per tile: 4 tokens per lane
-  const int n_tiles = len / kTileRows;
+  // one warp per tile: 4 tokens per lane; a ragged last tile is summarised over the tokens it has
+  const int n_tiles = tiles_of(len);
   const int tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31, bb = blockIdx.y;
   if (tile >= n_tiles) return;
   const int64_t base = (int64_t)bb * len + (int64_t)tile * kTileRows;
   int pmin = INT32_MAX, pmax = INT32_MIN, smin = INT32_MAX, smax = INT32_MIN, any = 0, all = 1, contig = 1;
   const int p0 = pos ? pos[base] : 0;
-  for (int e = lane; e < kTileRows; e += 32) {
+  const int n = min(kTileRows, len - tile * kTileRows);
+  for (int e = lane; e < n; e += 32) {
     if (pos) {
       int v = pos[base + e];
       pmin = min(pmin, v);
@@ -520,11 +539,11 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-template <int D>
+template <int D, bool RAGGED>
 cudaError_t launch_fwd(const FwdTcParams& P, cudaStream_t s) {
   constexpr size_t kSmem = 6 * kTileRows * D * 2 + kMaxTiles * 5 + NUM_BARS * 8 + 64 + 1024;
   constexpr size_t kRequest = kSmem < 120 * 1024 ? 120 * 1024 : kSmem;  // one CTA per SM: it owns all of TMEM
-  auto kern = tc_fwd_kernel<D>;
+  auto kern = tc_fwd_kernel<D, RAGGED>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRequest);
   if (e != cudaSuccess) return e;
   const int n_pairs = (P.n_q_tiles + 1) / 2;
@@ -605,7 +624,7 @@ bool make_tile_map(CUtensorMap* map, const TensorView& t, int b, int len, int h,
 
 cudaError_t launch_tile_meta(TileMeta* out, const int32_t* pos, const int32_t* seg, const uint8_t* pre, int b,
                              int len, cudaStream_t s) {
-  const int n_tiles = len / kTileRows;
+  const int n_tiles = tiles_of(len);
   dim3 grid((n_tiles + 7) / 8, b);
   tile_meta_kernel<<<grid, 256, 0, s>>>(out, pos, seg, pre, len);
   count_launch();
@@ -616,11 +635,10 @@ static bool aligned16(const TensorView& t) {
   return (reinterpret_cast<uintptr_t>(t.ptr) & 15) == 0 && (t.sb % 8) == 0 && (t.sl % 8) == 0 && (t.sh % 8) == 0;
 }
 
-const char* tc_fwd_unsupported_reason(const FwdParams& p, int dtype) {
+static const char* fwd_unsupported_reason(const FwdParams& p, int dtype) {
   if (dtype != RA_DTYPE_BF16) return "inputs are not bf16";
   if (p.dk != p.dv || (p.dk != 64 && p.dk != 128)) return "head dims must be equal and 64 or 128";
-  if (p.lq % kTileRows || p.lk % kTileRows) return "lq and lk must be multiples of 128";
-  if (p.lq / kTileRows > kMaxTiles || p.lk / kTileRows > kMaxTiles) return "more than 4096 tiles along one axis";
+  if (tiles_of(p.lq) > kMaxTiles || tiles_of(p.lk) > kMaxTiles) return "more than 4096 tiles along one axis";
   if ((p.mod.kinds & RA_MOD_DENSE) &&
       ((reinterpret_cast<uintptr_t>(p.mod.bias) & 15) || (p.mod.bsb % 4) || (p.mod.bsh % 4) || (p.mod.bsq % 4)))
     return "the dense bias needs a 16-byte aligned base and strides that are multiples of 4 floats";
@@ -630,12 +648,24 @@ const char* tc_fwd_unsupported_reason(const FwdParams& p, int dtype) {
   return nullptr;
 }
 
+const char* tc_fwd_unsupported_reason(const FwdParams& p, int dtype) {
+  if (p.lq % kTileRows || p.lk % kTileRows) return "lq and lk must be multiples of 128";
+  return fwd_unsupported_reason(p, dtype);
+}
+
+const char* tc_fwd_ragged_unsupported_reason(const FwdParams& p, int dtype) {
+  if (!(p.lq % kTileRows || p.lk % kTileRows)) return "lq and lk are multiples of 128";
+  if (!p.final_out.ptr || !p.first) return "ragged lengths are served for whole attentions with bf16 results";
+  if (p.mod.kinds & RA_MOD_DENSE) return "ragged lengths are not served with a dense bias tile";
+  return fwd_unsupported_reason(p, dtype);
+}
+
 cudaError_t tc_fwd_block(const FwdParams& p, cudaStream_t s) {
   FwdTcParams P;
   memset(&P, 0, sizeof(P));
   P.p = p;
-  P.n_q_tiles = p.lq / kTileRows;
-  P.n_kv_tiles = p.lk / kTileRows;
+  P.n_q_tiles = tiles_of(p.lq);
+  P.n_kv_tiles = tiles_of(p.lk);
   const char* why = nullptr;
   if (!make_tile_map(&P.map_q, p.q, p.b, p.lq, p.h, p.dk, kTileRows, &why) ||
       !make_tile_map(&P.map_k, p.k, p.b, p.lk, p.h, p.dk, kTileRows, &why) ||
@@ -655,7 +685,11 @@ cudaError_t tc_fwd_block(const FwdParams& p, cudaStream_t s) {
     P.meta_q = mq;
     P.meta_kv = mk;
   }
-  if (e == cudaSuccess) e = p.dk == 128 ? launch_fwd<128>(P, s) : launch_fwd<64>(P, s);
+  const bool ragged = p.lq % kTileRows || p.lk % kTileRows;
+  if (e == cudaSuccess) {
+    if (ragged) e = p.dk == 128 ? launch_fwd<128, true>(P, s) : launch_fwd<64, true>(P, s);
+    else e = p.dk == 128 ? launch_fwd<128, false>(P, s) : launch_fwd<64, false>(P, s);
+  }
   if (meta) cudaFreeAsync(meta, s);  // stream-ordered: after the kernels above, also when one failed to launch
   return e;
 }
@@ -770,7 +804,7 @@ extern "C" int ra_fwd_block_static(const ra_shape_t* shape, const ra_tensor_t* q
     P.meta_q = mq;
     P.meta_kv = mk;
   }
-  e = p.dk == 128 ? launch_fwd<128>(P, s) : launch_fwd<64>(P, s);
+  e = p.dk == 128 ? launch_fwd<128, false>(P, s) : launch_fwd<64, false>(P, s);
   if (e != cudaSuccess) return fail_cuda(e, "tcgen05 forward block (static scratch)");
   set_last_impl(RA_IMPL_TCGEN05);
   return 0;

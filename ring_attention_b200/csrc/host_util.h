@@ -21,6 +21,11 @@ int run_bwd_block(const BwdParams& p, int dtype, cudaStream_t s);
 // else a short text saying which condition failed.
 const char* tc_fwd_unsupported_reason(const FwdParams& p, int dtype);
 const char* tc_bwd_unsupported_reason(const BwdParams& p, int dtype);
+// The same for the forms that take lengths which are not multiples of 128 (a ring of one's whole
+// attention with bf16 results; see RAGGED in the kernels).  Used where no implementation was asked
+// for by name: block_impl "tcgen05" refuses such lengths.
+const char* tc_fwd_ragged_unsupported_reason(const FwdParams& p, int dtype);
+const char* tc_bwd_ragged_unsupported_reason(const BwdParams& p, int dtype);
 cudaError_t tc_fwd_block(const FwdParams& p, cudaStream_t s);
 cudaError_t tc_bwd_block(const BwdParams& p, cudaStream_t s);
 

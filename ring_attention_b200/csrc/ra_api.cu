@@ -92,6 +92,7 @@ int run_fwd_block(const FwdParams& p, int dtype, cudaStream_t s) {
   int impl = g_impl;
   if (impl != RA_IMPL_SIMT) {
     const char* why = tc_fwd_unsupported_reason(p, dtype);
+    if (why && impl == RA_IMPL_AUTO) why = tc_fwd_ragged_unsupported_reason(p, dtype);
     if (!why) {
       cudaError_t e = tc_fwd_block(p, s);
       if (e == cudaSuccess) {

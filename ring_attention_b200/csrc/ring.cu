@@ -536,11 +536,14 @@ void close_peers(ra_ring_t* r) {
 // Sizes of everything a ring call keeps in the handle, from the shape alone.
 struct RingSizes {
   size_t o_bytes, ml_bytes;                                // forward state
-  size_t delta_b, dq_b, dk_b, dv_b, own2_dk_b, own2_dv_b;  // backward accumulators
+  size_t delta_b, row_b, dq_b, dk_b, dv_b, own2_dk_b, own2_dv_b;  // backward accumulators
   bool split_b, split_h;  // the own backward block runs as two batch halves / head halves
   int b0, h0, nb2, nh2;
   size_t rows2;
 };
+
+// Rows per (batch, head) of the backward's row terms: whole 128-row tiles.
+int row_pitch(int lq) { return (lq + 127) / 128 * 128; }
 
 RingSizes ring_sizes(const ra_shape_t* shape, int nranks) {
   RingSizes z;
@@ -549,6 +552,7 @@ RingSizes ring_sizes(const ra_shape_t* shape, int nranks) {
   z.o_bytes = align_up(qrows * shape->dv * 4);
   z.ml_bytes = align_up(qrows * 4);
   z.delta_b = align_up(qrows * 4);
+  z.row_b = align_up((size_t)shape->b * shape->h * row_pitch(shape->lq) * 4);
   z.dq_b = align_up(qrows * shape->dk * 4);
   z.dk_b = align_up(krows * shape->dk * 4);
   z.dv_b = align_up(krows * shape->dv * 4);
@@ -1261,8 +1265,8 @@ BwdParams sub_problem(const BwdParams& p, int esize, int b0, int nb, int h0, int
   const int64_t bh0 = (int64_t)b0 * p.h + h0;
   s.lse = p.lse + bh0 * p.lq;
   s.delta = p.delta + bh0 * p.lq;
-  if (p.row_nl2) s.row_nl2 = p.row_nl2 + bh0 * p.lq;
-  if (p.row_nds) s.row_nds = p.row_nds + bh0 * p.lq;
+  if (p.row_nl2) s.row_nl2 = p.row_nl2 + bh0 * row_pitch(p.lq);
+  if (p.row_nds) s.row_nds = p.row_nds + bh0 * row_pitch(p.lq);
   s.dq = p.dq + bh0 * p.lq * p.dk_dim;
   s.dk = p.dk + bh0 * p.lk * p.dk_dim;
   s.dv = p.dv + bh0 * p.lk * p.dv_dim;
@@ -1313,10 +1317,10 @@ int ra_ring_bwd(ra_ring_t* ring, const ra_shape_t* shape, const ra_tensor_t* q,
   const int b0 = z.b0, h0 = z.h0, nb2 = z.nb2, nh2 = z.nh2;
   const size_t rows2 = z.rows2, own2_dk_b = z.own2_dk_b, own2_dv_b = z.own2_dv_b;
   // delta, then the two per-row terms derived from L and delta that the tensor-core kernel reads
-  RA_CUDA(ring->grads.reserve(3 * delta_b + dq_b + dk_b + dv_b + own2_dk_b + own2_dv_b), "cudaMalloc(grads)");
-  char* g = (char*)ring->grads.ptr + 2 * delta_b;
+  RA_CUDA(ring->grads.reserve(2 * z.row_b + delta_b + dq_b + dk_b + dv_b + own2_dk_b + own2_dv_b), "cudaMalloc(grads)");
+  char* g = (char*)ring->grads.ptr + 2 * z.row_b;
   float* row_nl2 = (float*)ring->grads.ptr;
-  float* row_nds = (float*)((char*)ring->grads.ptr + delta_b);
+  float* row_nds = (float*)((char*)ring->grads.ptr + z.row_b);
   float* delta = (float*)g;
   float* dq_acc = (float*)(g + delta_b);
   float* dk_acc = (float*)(g + delta_b + dq_b);
@@ -1337,7 +1341,7 @@ int ra_ring_bwd(ra_ring_t* ring, const ra_shape_t* shape, const ra_tensor_t* q,
   if (e != cudaSuccess) return fail_cuda(e, "delta");
   p.delta = delta;
   if (current_impl() != RA_IMPL_SIMT) {  // once per backward, not once per block launch
-    e = launch_bwd_row_terms(lse, delta, shape->sm_scale, 1, (int64_t)shape->b * shape->h * shape->lq, row_nl2, row_nds, stream);
+    e = launch_bwd_row_terms(lse, delta, shape->sm_scale, 1, (int64_t)shape->b * shape->h, shape->lq, row_pitch(shape->lq), row_nl2, row_nds, stream);
     if (e != cudaSuccess) return fail_cuda(e, "row terms");
     p.row_nl2 = row_nl2;
     p.row_nds = row_nds;
@@ -1352,7 +1356,8 @@ int ra_ring_bwd(ra_ring_t* ring, const ra_shape_t* shape, const ra_tensor_t* q,
   if (N == 1 && current_impl() != RA_IMPL_SIMT && !(p.mod.kinds & RA_MOD_STRICT_NAN)) {
     p.dk_out = tv(dk);
     p.dv_out = tv(dv);
-    direct = tc_bwd_unsupported_reason(p, shape->dtype) == nullptr;
+    direct = tc_bwd_unsupported_reason(p, shape->dtype) == nullptr ||
+             (current_impl() == RA_IMPL_AUTO && tc_bwd_ragged_unsupported_reason(p, shape->dtype) == nullptr);
     if (!direct) p.dk_out = p.dv_out = TensorView{nullptr, 0, 0, 0};
   }
   RA_CUDA(cudaMemsetAsync(dq_acc, 0, direct ? dq_b : dq_b + dk_b + dv_b, stream), "cudaMemsetAsync");
@@ -1566,7 +1571,7 @@ int ra_ring_reserve(ra_ring_t* ring, const ra_shape_t* shape, const ra_score_mod
   const KvMessage msg = make_kv_message(shape, none, none, m);
   RA_CUDA(ring->state.reserve(z.o_bytes + 2 * z.ml_bytes), "cudaMalloc(state)");
   if (backward) {
-    RA_CUDA(ring->grads.reserve(3 * z.delta_b + z.dq_b + z.dk_b + z.dv_b + z.own2_dk_b + z.own2_dv_b), "cudaMalloc(grads)");
+    RA_CUDA(ring->grads.reserve(2 * z.row_b + z.delta_b + z.dq_b + z.dk_b + z.dv_b + z.own2_dk_b + z.own2_dv_b), "cudaMalloc(grads)");
     if (N > 1)
       for (int i = 0; i < kSlots; ++i) RA_CUDA(ring->part[i].reserve(z.dk_b + z.dv_b), "cudaMalloc(part)");
   }

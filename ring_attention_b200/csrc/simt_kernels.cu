@@ -622,13 +622,23 @@ cudaError_t launch_strict_nan(int b, int h, int lq, int lk, int dk_dim, int dv_d
   return cudaGetLastError();
 }
 
+// Rows are padded from lq to `pitch` per (batch, head); a padding row gets P = 0 and dS = 0.
 __global__ void bwd_row_terms_kernel(const float* __restrict__ lse, const float* __restrict__ delta, float scale,
-                                     int clamp, int64_t n, float* __restrict__ nl2, float* __restrict__ nds) {
+                                     int clamp, int64_t n, int lq, int pitch, float* __restrict__ nl2,
+                                     float* __restrict__ nds) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const float x = -lse[i] * 1.4426950408889634f;
+  const int64_t bh = i / pitch;
+  const int r = (int)(i - bh * pitch);
+  if (r >= lq) {
+    nl2[i] = -1e30f;
+    nds[i] = 0.f;
+    return;
+  }
+  const float L = lse[bh * lq + r], x = -L * 1.4426950408889634f;
   nl2[i] = clamp ? fminf(x, 1e30f) : x;
-  nds[i] = -delta[i] * scale;
+  // a row that saw no key has delta = NaN; without a dense bias it contributes nothing
+  nds[i] = (clamp && L == -INFINITY) ? 0.f : -delta[bh * lq + r] * scale;
 }
 
 __global__ void add_rows_f32_kernel(float* __restrict__ dst, const float* __restrict__ src, int64_t seg_elems,
@@ -643,9 +653,10 @@ __global__ void add_rows_f32_kernel(float* __restrict__ dst, const float* __rest
   }
 }
 
-cudaError_t launch_bwd_row_terms(const float* lse, const float* delta, float scale, int clamp, int64_t n, float* nl2,
-                                 float* nds, cudaStream_t s) {
-  bwd_row_terms_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(lse, delta, scale, clamp, n, nl2, nds);
+cudaError_t launch_bwd_row_terms(const float* lse, const float* delta, float scale, int clamp, int64_t bh, int lq,
+                                 int pitch, float* nl2, float* nds, cudaStream_t s) {
+  const int64_t n = bh * pitch;
+  bwd_row_terms_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(lse, delta, scale, clamp, n, lq, pitch, nl2, nds);
   count_launch();
   return cudaGetLastError();
 }

@@ -10,6 +10,7 @@ namespace ra {
 
 constexpr int kTileRows = 128;     // rows of one q tile / one kv tile
 constexpr int kMaxTiles = 4096;    // most tiles one block (shard) may have along either axis
+__host__ __device__ constexpr int tiles_of(int rows) { return (rows + kTileRows - 1) / kTileRows; }
 
 constexpr uint32_t kMaskKinds = RA_MOD_CAUSAL | RA_MOD_SEGMENT | RA_MOD_PREFIX | RA_MOD_WINDOW;
 // Score-mods that read the tile summaries (ALiBi reads pos_contig to choose its in-loop form).
@@ -20,6 +21,14 @@ __device__ __forceinline__ uint32_t bits_from(int first) {
   return first <= 0 ? 0xffffffffu : (first >= 32 ? 0u : 0xffffffffu << first);
 }
 __device__ __forceinline__ uint32_t bits_below(int last) { return ~bits_from(last); }
+
+// The bf16 pair in `hi` (the rounded x0, x1) leaves a remainder; this is that remainder as a second
+// bf16 pair: hi + lo holds 16 bits of each value.  A value that rounded to infinity keeps lo = 0.
+__device__ __forceinline__ uint32_t pack_bf16_rest(uint32_t hi, float x0, float x1) {
+  const float h0 = __uint_as_float(hi << 16), h1 = __uint_as_float(hi & 0xffff0000u);
+  const float r0 = fabsf(h0) == INFINITY ? 0.f : x0 - h0, r1 = fabsf(h1) == INFINITY ? 0.f : x1 - h1;
+  return ptx::pack_bf16(r0, r1);
+}
 
 // Which of the 32 * kWords columns of a tile this thread's row sees under the mask kinds: bit c of
 // the words = column c.  kRowIsQuery: the row is a query and the columns are keys (forward); else
@@ -35,13 +44,15 @@ __device__ __forceinline__ uint32_t bits_below(int last) { return ~bits_from(las
 //   * scattered positions: one shuffle and compare per column.
 // (The form before this one evaluated the mask per pair on scores in TMEM: about 17,000 cycles for
 // a 128 x 128 forward tile, several times the rest of the tile's softmax.)
-// All 32 lanes of the warp call it; the column arrays point at the tile's first column.
+// All 32 lanes of the warp call it; the column arrays point at the tile's first column and hold `ncols`
+// entries from there: columns past them (a ragged last tile) are not read and count as masked.
 template <bool kRowIsQuery, int kWords>
 __device__ __forceinline__ void visible_columns(uint32_t (&vis)[kWords], uint32_t kinds, int32_t window, int32_t row_pos,
                                                 int32_t row_seg, bool row_pre, const int32_t* col_pos,
                                                 const int32_t* col_seg, const uint8_t* col_pre, int32_t col_pos0,
-                                                bool col_contig) {
+                                                bool col_contig, int ncols = 32 * kWords) {
   const int lane = threadIdx.x & 31;
+  auto col = [&](int w) { return min(32 * w + lane, ncols - 1); };  // this lane's column of word w, kept inside
   const bool order = (kinds & (RA_MOD_CAUSAL | RA_MOD_PREFIX)) != 0, win = (kinds & RA_MOD_WINDOW) != 0;
   if (!(order || win)) {
 #pragma unroll
@@ -65,7 +76,7 @@ __device__ __forceinline__ void visible_columns(uint32_t (&vis)[kWords], uint32_
     for (int w = 0; w < kWords; ++w) {
       uint32_t m = bits_from(f - 32 * w) & bits_below(l - 32 * w);
       if (kinds & RA_MOD_PREFIX) {
-        const uint32_t pre = __ballot_sync(0xffffffffu, col_pre[32 * w + lane] != 0);
+        const uint32_t pre = __ballot_sync(0xffffffffu, col_pre[col(w)] != 0);
         if (row_pre) m |= pre;
       }
       vis[w] = m & bits_from(wf - 32 * w) & bits_below(wl - 32 * w);
@@ -73,7 +84,7 @@ __device__ __forceinline__ void visible_columns(uint32_t (&vis)[kWords], uint32_
   } else {
 #pragma unroll
     for (int w = 0; w < kWords; ++w) {
-      const int32_t cp = col_pos[32 * w + lane];
+      const int32_t cp = col_pos[col(w)];
       uint32_t m = 0xffffffffu, near = 0xffffffffu;
 #pragma unroll 1
       for (int c = 0; c < 32; ++c) {
@@ -83,7 +94,7 @@ __device__ __forceinline__ void visible_columns(uint32_t (&vis)[kWords], uint32_
         if (win && qp - kp >= window) near &= ~(1u << c);
       }
       if (kinds & RA_MOD_PREFIX) {
-        const uint32_t pre = __ballot_sync(0xffffffffu, col_pre[32 * w + lane] != 0);
+        const uint32_t pre = __ballot_sync(0xffffffffu, col_pre[col(w)] != 0);
         if (row_pre) m |= pre;
       }
       vis[w] = m & near;
@@ -92,7 +103,7 @@ __device__ __forceinline__ void visible_columns(uint32_t (&vis)[kWords], uint32_
   if (kinds & RA_MOD_SEGMENT) {
     int32_t cs[kWords];
 #pragma unroll
-    for (int w = 0; w < kWords; ++w) cs[w] = col_seg[32 * w + lane];
+    for (int w = 0; w < kWords; ++w) cs[w] = col_seg[col(w)];
     uint32_t todo = 0xffffffffu;  // rows of the warp whose id has not been looked up yet
 #pragma unroll 1
     while (todo) {
@@ -106,6 +117,8 @@ __device__ __forceinline__ void visible_columns(uint32_t (&vis)[kWords], uint32_
       todo &= ~__ballot_sync(0xffffffffu, mine);
     }
   }
+#pragma unroll
+  for (int w = 0; w < kWords; ++w) vis[w] &= bits_below(ncols - 32 * w);
 }
 
 // Adds a per-pair bias to raw (unscaled) scores that sit in TMEM, in place: this thread's TMEM
@@ -118,11 +131,11 @@ __device__ __forceinline__ void visible_columns(uint32_t (&vis)[kWords], uint32_
 // kRowIsQuery: as above.  `bias` points at this thread's row and the tile's first column,
 // consecutive columns are `bias_col_stride` floats apart (1 in the forward, where a thread reads
 // 64 contiguous bytes per 16 columns; the bias row stride in the backward, where the lanes of a
-// warp read consecutive floats of one bias row).
+// warp read consecutive floats of one bias row).  `ncols_valid`: positions past it are not read.
 template <bool kRowIsQuery>
 __device__ __noinline__ void bias_scores_tmem(uint32_t taddr, int ncols, bool alibi, float alibi_over_scale,
                                               int32_t row_pos, const int32_t* col_pos, const float* bias,
-                                              int64_t bias_col_stride, float inv_scale) {
+                                              int64_t bias_col_stride, float inv_scale, int ncols_valid) {
   uint32_t cur[16], nxt[16];
   ptx::tmem_ld16(taddr, cur);
 #pragma unroll 1
@@ -148,7 +161,7 @@ __device__ __noinline__ void bias_scores_tmem(uint32_t taddr, int ncols, bool al
     if (alibi) {
 #pragma unroll
       for (int e = 0; e < 16; ++e) {
-        const int32_t cp = __ldg(col_pos + c0 + e);
+        const int32_t cp = __ldg(col_pos + min(c0 + e, ncols_valid - 1));
         const int32_t dist = kRowIsQuery ? row_pos - cp : cp - row_pos;  // q_pos - kv_pos
         cur[e] = __float_as_uint(fmaf(-alibi_over_scale, (float)dist, __uint_as_float(cur[e])));
       }
