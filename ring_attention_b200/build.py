@@ -15,7 +15,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libring_attention_b200.so")
-SOURCES = ["ra_api.cu", "ring.cu", "simt_kernels.cu", "fwd_sm100.cu", "bwd_sm100.cu"]
+SOURCES = ["ra_api.cu", "ring.cu", "simt_kernels.cu", "simt_wide.cu", "fwd_sm100.cu", "bwd_sm100.cu"]
 
 
 def _nccl_include() -> str:

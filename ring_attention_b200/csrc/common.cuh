@@ -75,6 +75,9 @@ struct BwdParams {
 // Launchers implemented in the .cu files.  Each returns a cudaError_t.
 cudaError_t simt_fwd_block(const FwdParams& p, int dtype, cudaStream_t s);
 cudaError_t simt_bwd_block(const BwdParams& p, int dtype, cudaStream_t s);
+// Head dims 17 to 128 of the two above.
+cudaError_t simt_wide_fwd(const FwdParams& p, int dtype, cudaStream_t s);
+cudaError_t simt_wide_bwd(const BwdParams& p, int dtype, cudaStream_t s);
 // out = o / l, L = m + log l (ring.py:134-135).  With o2 != NULL the two carried states are
 // merged first, as one more online-softmax update (ring.py:63-75) would.
 cudaError_t launch_finalize(int b, int h, int lq, int dv, const float* o, const float* m, const float* l,

@@ -2,7 +2,9 @@
 // attention), any score-mod including a dense bias tile, fp32 or bf16 inputs with all
 // arithmetic in fp32.  They are the exact path (1e-5 against an fp64 restatement of
 // ring_attention/ring.py:58-76 and :140-157) and serve every shape the tcgen05 kernels
-// do not take.
+// do not take.  The kernels of this file serve head dims up to 16 (a quarter of the padded
+// columns of the wide kernels) and above 128 (whose tiles do not fit in shared memory whole);
+// the ones between go to simt_wide.cu.
 #include <math.h>
 
 #include "common.cuh"
@@ -556,25 +558,26 @@ template <typename T>
 cudaError_t dispatch_fwd(const FwdParams& p, cudaStream_t s) {
   int d = p.dv;
   if (d <= 16) return launch_fwd<T, 16>(p, s);
-  if (d <= 64) return launch_fwd<T, 64>(p, s);
-  if (d <= 128) return launch_fwd<T, 128>(p, s);
   return launch_fwd<T, 256>(p, s);
 }
 template <typename T>
 cudaError_t dispatch_bwd(const BwdParams& p, cudaStream_t s) {
   int d = p.dk_dim > p.dv_dim ? p.dk_dim : p.dv_dim;
   if (d <= 16) return launch_bwd<T, 16>(p, s);
-  if (d <= 64) return launch_bwd<T, 64>(p, s);
-  if (d <= 128) return launch_bwd<T, 128>(p, s);
   return launch_bwd<T, 256>(p, s);
 }
 
 }  // namespace
 
+// Whether simt_wide.cu serves these head dims.
+static bool wide(int dk, int dv) { return (dk > 16 || dv > 16) && dk <= 128 && dv <= 128; }
+
 cudaError_t simt_fwd_block(const FwdParams& p, int dtype, cudaStream_t s) {
+  if (wide(p.dk, p.dv)) return simt_wide_fwd(p, dtype, s);
   return dtype == RA_DTYPE_F32 ? dispatch_fwd<float>(p, s) : dispatch_fwd<__nv_bfloat16>(p, s);
 }
 cudaError_t simt_bwd_block(const BwdParams& p, int dtype, cudaStream_t s) {
+  if (wide(p.dk_dim, p.dv_dim)) return simt_wide_bwd(p, dtype, s);
   return dtype == RA_DTYPE_F32 ? dispatch_bwd<float>(p, s) : dispatch_bwd<__nv_bfloat16>(p, s);
 }
 
