@@ -56,15 +56,6 @@ constexpr int bwd_threads(bool drain) { return drain ? 512 : 320; }
 // compute warps, one drain warp and one of the others, 2 * 152 + 152 + 56 = 512 = 16384 / 32.
 constexpr int kRegsCompute = 152, kRegsDrain = 152, kRegsOther = 56;
 
-template <int N>
-__device__ __forceinline__ void reg_inc() {
-  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
-}
-template <int N>
-__device__ __forceinline__ void reg_dec() {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
-}
-
 __host__ __device__ constexpr int bwd_do_stages(int d, bool ragged) { return ragged && d == 128 ? 1 : 2; }
 
 constexpr float kLog2e = 1.4426950408889634f;

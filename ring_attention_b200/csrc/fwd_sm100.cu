@@ -33,15 +33,19 @@ namespace {
 
 using namespace ptx;
 
-constexpr int kFwdThreads = 320;
+// Three whole warpgroups (two of softmax; producer, MMA issuer and two idle warps), so that registers
+// can be re-divided between them: every scheduler hosts two softmax warps and one of the others,
+// 2 * 216 + 72 = 504 = 3 * 168 of the 512 per lane that a scheduler has.  A softmax thread holds 128
+// scores: with 168 registers (320 threads, no re-division) its chains were cut short by spills and
+// waits.  Unmasked 8k tokens, d 128: 1003 -> 933 us; causal: 567 -> 517 us.
+constexpr int kFwdThreads = 384, kRegsSoftmax = 216, kRegsOther = 72;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kRescaleThreshold = 8.0f;  // log2 units: P stays below 2^8
 // Of every 16 column pairs of the softmax, how many get their exponentials from the polynomial
-// on the FMA pipe (the others use ex2 on the special-function unit).
-#ifndef RA_FWD_POLY_PAIRS
-#define RA_FWD_POLY_PAIRS 5
-#endif
-constexpr int kPolyPairs = RA_FWD_POLY_PAIRS;
+// on the FMA pipe (the others use ex2 on the special-function unit).  Forward of 32k causal tokens,
+// d 128, with 0 / 2 / 3 / 4 / 5 / 6 pairs: 7.85 / 7.99 / 7.55 / 7.44 / 8.55 / 8.07 ms; of 64k windowed
+// tokens, d 64: 7.63 / 7.70 / 7.78 / 7.81 / 8.02 / 8.61 ms (tiles with half the MMA time gain nothing).
+__host__ __device__ constexpr int poly_pairs(int d) { return d == 128 ? 4 : 0; }
 
 struct FwdTcParams {
   CUtensorMap map_q, map_k, map_v;
@@ -68,6 +72,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
   constexpr int TILE_BYTES = kTileRows * D * 2;
   constexpr int PANELS = D / 64;           // 64-element (128-byte) panels per row
   constexpr int PANEL_BYTES = kTileRows * 128;
+  constexpr int kPolyPairs = RAGGED ? 0 : poly_pairs(D);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;
@@ -161,7 +166,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
   const uint32_t tmem_S[2] = {tmem_base, tmem_base + 128};
   const uint32_t tmem_O[2] = {tmem_base + 256, tmem_base + 256 + D};
 
-  if (warp == 8) {
+  if (warp >= 8) {
+    reg_dec<kRegsOther>();
+    if (warp == 8) {
     // ------------------------------------------------------------ TMA producer
     if (lane == 0) {
       prefetch_tensormap(&P.map_q);
@@ -188,7 +195,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
                       j * kTileRows, bb);
       }
     }
-  } else if (warp == 9) {
+    } else if (warp == 9) {
     // ------------------------------------------------------------ MMA issuer
     if (count > 0) {  // every lane runs this loop; one elected lane issues each instruction
       constexpr uint32_t idesc_qk = make_idesc_bf16(128, 128, false, false);
@@ -251,7 +258,10 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
       }
       if (ok) tc_commit_warp(&bars[O_FULL]);
     }
-  } else if (warp < 4 * ntile) {
+    }
+  } else {
+    reg_inc<kRegsSoftmax>();
+    if (warp < 4 * ntile) {
     // ------------------------------------------------------------ softmax + epilogue
     const int t = warp >> 2;
     const int row_in_tile = (warp & 3) * 32 + lane;
@@ -374,7 +384,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
         for (int e = 0; e < 16; ++e) {
           const uint64_t x2 = fma2(pack2(__uint_as_float(r[c][2 * e]), __uint_as_float(r[c][2 * e + 1])), sc2, nm2);
           float p0, p1;
-          if (!RAGGED && e < kPolyPairs) {
+          if (e < kPolyPairs) {
             exp2_poly2(x2, p0, p1);
           } else {
             float x0, x1;
@@ -453,6 +463,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
         p.m[state_row] = m_true * (1.f / kLog2e);
         p.l[state_row] = l_tot;
       }
+    }
     }
   }
 

@@ -230,6 +230,16 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// Registers per thread of this warpgroup from here on (all four warps execute it).
+template <int N>
+__device__ __forceinline__ void reg_inc() {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+}
+template <int N>
+__device__ __forceinline__ void reg_dec() {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
+}
+
 // ---- packed fp32 pairs and other arithmetic helpers of the softmax loops ---------------------
 // Two floats in one 64-bit register pair: fma / add on both halves in one instruction.
 __device__ __forceinline__ uint64_t pack2(float lo, float hi) {
