@@ -15,13 +15,12 @@
 //           the softmax scale rides on dS^T, so dQ and dK need no further scaling)
 //   dV  += P^T dO         (TS MMA: A from TMEM, B = dO read MN-major) -> TMEM [256,256+D)
 //   dK  += dS^T Q         (SS MMA: B = Q read MN-major)               -> TMEM [256+D,256+2D)
-//   dQ^T = K^T dS^T       (SS MMA: A = K read MN-major, B = dS^T tile read MN-major; head dim 128)
-//                          -> TMEM [128,256), over dP^T; lane = head-dim index.  A warpgroup of
+//   dQ^T = K^T dS^T       (SS MMA: A = K read MN-major, B = dS^T tile read MN-major)
+//                          -> TMEM [128,256), over dP^T (head dim 64: [384,512)); lane = head-dim index.  A warpgroup of
 //                             its own takes the whole tile into registers, hands the columns
 //                             back, and adds the values to the fp32 accumulator with one
 //                             reduction per query column: a warp's instruction covers 128
 //                             contiguous bytes of a dQ row.
-//                             (head dim 64 forms dQ = dS K instead; the compute warps reduce it.)
 // Shared-memory bandwidth bounds this kernel: an SS MMA of 128 x 128 x 16 reads 8 KB of operands
 // in the 64 cycles its arithmetic takes, which is all of the 128 bytes per cycle that shared
 // memory delivers, so every other access on that data path (TMA writes of Q and dO, the dS^T
@@ -33,9 +32,8 @@
 // halves each (P^T hi and lo in the two halves of a warpgroup's S^T columns, dS^T in two shared-memory
 // tiles), and dV, dK and dQ take two MMAs per k-step.  At head dim 128 the second dS^T tile takes the
 // room of the second dO stage.
-// Head dim 128: warps 0-7 compute (two warpgroups split the 128 query columns), warps 8-11 drain
-// dQ^T, warp 12 TMA producer, warp 13 MMA issuer, warps 14-15 idle (registers are re-divided
-// between whole warpgroups).  Head dim 64: warps 0-7 compute, warp 8 producer, warp 9 MMA issuer.
+// Warps 0-7 compute (two warpgroups split the 128 query columns), warps 8-11 drain dQ^T, warp 12 TMA
+// producer, warp 13 MMA issuer, warps 14-15 idle (registers are re-divided between whole warpgroups).
 // Grid: CTAs of a few (batch, head) pairs at a time, so that the Q / dO tiles and the dQ
 // accumulator rows that the resident CTAs stream stay in L2.
 #include <cstdio>
@@ -50,10 +48,9 @@ namespace {
 
 using namespace ptx;
 
-// 10 warps; with the drain warpgroup (head dim 128) 16
-constexpr int bwd_threads(bool drain) { return drain ? 512 : 320; }
-// Registers per thread after the re-division, with the drain warpgroup: every scheduler hosts two
-// compute warps, one drain warp and one of the others, 2 * 152 + 152 + 56 = 512 = 16384 / 32.
+constexpr int kBwdThreads = 512;  // four warpgroups: two of compute, the drain, the other roles
+// Registers per thread after the re-division: every scheduler hosts two compute warps, one drain
+// warp and one of the others, 2 * 152 + 152 + 56 = 512 = 16384 / 32.
 constexpr int kRegsCompute = 152, kRegsDrain = 152, kRegsOther = 56;
 
 __host__ __device__ constexpr int bwd_do_stages(int d, bool ragged) { return ragged && d == 128 ? 1 : 2; }
@@ -83,28 +80,29 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint
       : "memory");
 }
 
-__device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d)
-               : "memory");
-}
-
 template <int D, bool RAGGED>
-__global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const __grid_constant__ BwdTcParams P) {
-  constexpr bool DRAIN = D == 128;  // the drain warpgroup serves the dQ^T form
-  constexpr int PRODUCER_WARP = DRAIN ? 12 : 8, MMA_WARP = PRODUCER_WARP + 1;
+__global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_constant__ BwdTcParams P) {
+  constexpr int PRODUCER_WARP = 12, MMA_WARP = 13;
+  // Head dim 64 leaves tensor memory for columns of dQ^T's own: dP^T of the next tile need not wait
+  // until dQ^T has been drained.  It is then issued before the MMAs that read dS^T, so dS^T has two stages.
+  // Unmasked 8k tokens, d 64: 3.25 -> 2.40 ms (with dQ formed untransposed, drained by the compute
+  // warps and sharing dP^T's columns before); what bounds it now is the compute warps' own work.
+  constexpr bool SEP_DQ = D == 64;
+  constexpr int DS_ST = SEP_DQ ? 2 : 1;
   constexpr int TILE_BYTES = kTileRows * D * 2;
   constexpr int PANELS = D / 64;
   constexpr int PANEL_BYTES = kTileRows * 128;
   constexpr int DS_BYTES = kTileRows * kTileRows * 2;
   constexpr int DO_ST = bwd_do_stages(D, RAGGED);
   constexpr int DS_TILES = RAGGED ? 2 : 1;  // dS^T, and what its rounding to bf16 left
+  constexpr int DS_STAGE_BYTES = DS_TILES * DS_BYTES;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sK = smem;
   uint8_t* sV = sK + TILE_BYTES;
   uint8_t* sQ = sV + TILE_BYTES;          // 2 stages
   uint8_t* sdO = sQ + 2 * TILE_BYTES;     // DO_ST stages
-  uint8_t* sdS = sdO + DO_ST * TILE_BYTES;  // [128 key rows][128 query cols] bf16, 2 panels, 128B swizzle
-  float* sL = reinterpret_cast<float*>(sdS + DS_TILES * DS_BYTES);  // [2][128]
+  uint8_t* sdS = sdO + DO_ST * TILE_BYTES;  // DS_ST stages of [128 key rows][128 query cols] bf16, 2 panels, 128B swizzle
+  float* sL = reinterpret_cast<float*>(sdS + DS_ST * DS_STAGE_BYTES);  // [2][128]
   float* sDelta = sL + 2 * kTileRows;                     // [2][128]
   uint64_t* bars = reinterpret_cast<uint64_t*>(sDelta + 2 * kTileRows);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NUM_BARS);
@@ -127,7 +125,7 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < NUM_BARS; ++i) {
-      uint32_t cnt = (i == P_READY || i == DS_READY) ? 256u : (i == DQ_DRAINED) ? (DRAIN ? 128u : 256u) : 1u;
+      uint32_t cnt = (i == P_READY || i == DS_READY) ? 256u : (i == DQ_DRAINED) ? 128u : 1u;
       mbar_init(&bars[i], cnt);
     }
     *abort_flag = (smem_u32(smem) & 1023u) ? 1u : 0u;  // the swizzled tiles need a 1024-byte aligned base
@@ -190,15 +188,15 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
   tc_fence_after();
   const uint32_t tmem_base = has_work ? __shfl_sync(0xffffffffu, *tmem_slot, 0) : 0u;
   const uint32_t tmem_S = tmem_base, tmem_dP = tmem_base + 128, tmem_dV = tmem_base + 256,
-                 tmem_dK = tmem_base + 256 + D;
+                 tmem_dK = tmem_base + 256 + D, tmem_dQ = SEP_DQ ? tmem_base + 256 + 2 * D : tmem_dP;
   const bool bad = *abort_flag != 0;
 
   if (bad) {
     // fall through to the common exit
   } else if (warp >= PRODUCER_WARP) {
-    // the producer warp and the MMA warp; with the drain warpgroup they and two idle warps form
-    // a warpgroup, which hands most of its registers to the others
-    if constexpr (DRAIN) reg_dec<kRegsOther>();
+    // the producer warp, the MMA warp and two idle warps form a warpgroup, which hands most of its
+    // registers to the others
+    reg_dec<kRegsOther>();
     if (warp == PRODUCER_WARP) {
     // ------------------------------------------------------------ TMA producer
     // The whole warp walks the tile sequence (the scan is warp-wide); lane 0 polls and issues.
@@ -281,13 +279,16 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
       // every lane runs this loop; one elected lane issues each instruction
       constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);   // S^T, dP^T
       constexpr uint32_t idesc_dv = make_idesc_bf16(128, D, false, true);     // dV, dK: B MN-major
-      // dQ: A and B MN-major.  D = 128 forms dQ^T (M = D, N = 128 queries); D = 64 forms dQ (M = 128 queries, N = D)
-      constexpr uint32_t idesc_dq = make_idesc_bf16(128, D == 128 ? 128 : D, true, true);
+      // dQ^T: A and B MN-major, M = head dim, N = 128 queries.  At head dim 64 A's two 64-row panels are
+      // the same one (panels 0 bytes apart): lanes 64 to 127 hold the 64 rows again, so that all four
+      // drain warps have lanes to read, two of them for each half of the queries.
+      constexpr uint32_t idesc_dq = make_idesc_bf16(128, 128, true, true);
+      constexpr uint32_t kDsStage16 = DS_STAGE_BYTES >> 4;
       // Low descriptor words: K-major views step 32 B per k-step inside a 64-column panel and one
       // panel (16 KB) per 4 k-steps; MN-major views step 16 rows (2 KB) per k-step, panels 16 KB apart.
       constexpr uint32_t kPanel16 = PANEL_BYTES >> 4, kStage16 = TILE_BYTES >> 4;
       constexpr uint32_t kLow16 = DS_BYTES >> 4;  // from a dS^T tile to its low half
-      const uint32_t k_km = desc_lo(smem_u32(sK), 16), k_mn = desc_lo(smem_u32(sK), PANEL_BYTES);
+      const uint32_t k_km = desc_lo(smem_u32(sK), 16), k_mn = desc_lo(smem_u32(sK), D == 128 ? PANEL_BYTES : 0);
       const uint32_t v_km = desc_lo(smem_u32(sV), 16);
       const uint32_t q_km = desc_lo(smem_u32(sQ), 16), q_mn = desc_lo(smem_u32(sQ), PANEL_BYTES);
       const uint32_t do_km = desc_lo(smem_u32(sdO), 16), do_mn = desc_lo(smem_u32(sdO), PANEL_BYTES);
@@ -324,7 +325,8 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
       // Issue order per query tile n (the tensor pipe executes in this order):
       //   S(n+1) | dQ(n) | dK(n) | dP(n+1) | dV(n+1)
       // so that the compute warps form P(n+1) under dQ(n)/dK(n), drain dQ(n) under dK(n), and
-      // form dS(n+1) under dV(n+1)/S(n+2).
+      // form dS(n+1) under dV(n+1)/S(n+2).  With dQ in columns of its own dP(n+1) goes before dQ(n):
+      // the compute warps then have both their inputs waiting and never stand still for the pipe.
       bool ok = true;
       Window& win = win0;
       int i = first_tile;
@@ -355,49 +357,53 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
             tc_fence_after();
             issue_s(sn);
           }
-          // dQ = dS K (into the dP^T columns), dK += dS^T Q
+          // dQ^T = K^T dS^T, dK += dS^T Q
           if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[DS_READY], par, abort_flag, P.status, kStBwdMma)))) break;
           tc_fence_after();
-          if constexpr (D == 128) {
-            // dQ^T = K^T dS^T: lane = head-dim index, column = query, so that a warp's reduction
-            // instruction covers 128 contiguous bytes of one dQ row
-#pragma unroll
-            for (int kk = 0; kk < 8; ++kk)
-              mma_ss_warp(tmem_dP, desc_from_lo(k_mn + mn_off(kk)), desc_from_lo(ds_mn + mn_off(kk)), idesc_dq, kk > 0);
-            if constexpr (RAGGED) {
-#pragma unroll
-              for (int kk = 0; kk < 8; ++kk)
-                mma_ss_warp(tmem_dP, desc_from_lo(k_mn + mn_off(kk)), desc_from_lo(ds_mn + kLow16 + mn_off(kk)), idesc_dq, 1u);
+          if constexpr (SEP_DQ) {
+            if (has_next) {  // the compute warps have read dP(n)
+              if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[DO_FULL0 + dsn], dphn, abort_flag, P.status, kStBwdMma)))) break;
+              tc_fence_after();
+              issue_dp(dsn);
             }
-          } else {
+            if (n > 0 && !(ok = __all_sync(0xffffffffu, mbar_wait(&bars[DQ_DRAINED], par ^ 1, abort_flag, P.status, kStBwdMma)))) break;
+            tc_fence_after();
+          }
+          const uint32_t ds0 = (n % DS_ST) * kDsStage16;
+          {
+            // lane = head-dim index, column = query, so that a warp's reduction instruction covers
+            // 128 contiguous bytes of one dQ row
+            const uint32_t b0 = ds_mn + ds0;
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk)
-              mma_ss_warp(tmem_dP, desc_from_lo(ds_mn + mn_off(kk)), desc_from_lo(k_mn + mn_off(kk)), idesc_dq, kk > 0);
+              mma_ss_warp(tmem_dQ, desc_from_lo(k_mn + mn_off(kk)), desc_from_lo(b0 + mn_off(kk)), idesc_dq, kk > 0);
             if constexpr (RAGGED) {
 #pragma unroll
               for (int kk = 0; kk < 8; ++kk)
-                mma_ss_warp(tmem_dP, desc_from_lo(ds_mn + kLow16 + mn_off(kk)), desc_from_lo(k_mn + mn_off(kk)), idesc_dq, 1u);
+                mma_ss_warp(tmem_dQ, desc_from_lo(k_mn + mn_off(kk)), desc_from_lo(b0 + kLow16 + mn_off(kk)), idesc_dq, 1u);
             }
           }
           tc_commit_warp(&bars[DQ_FULL]);
           {
-            const uint32_t b0 = q_mn + s * kStage16;
+            const uint32_t a0 = ds_km + ds0, b0 = q_mn + s * kStage16;
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk)
-              mma_ss_warp(tmem_dK, desc_from_lo(ds_km + km_off(kk)), desc_from_lo(b0 + mn_off(kk)), idesc_dv,
+              mma_ss_warp(tmem_dK, desc_from_lo(a0 + km_off(kk)), desc_from_lo(b0 + mn_off(kk)), idesc_dv,
                      (n > 0) || kk > 0);
             if constexpr (RAGGED) {
 #pragma unroll
               for (int kk = 0; kk < 8; ++kk)
-                mma_ss_warp(tmem_dK, desc_from_lo(ds_km + kLow16 + km_off(kk)), desc_from_lo(b0 + mn_off(kk)), idesc_dv, 1u);
+                mma_ss_warp(tmem_dK, desc_from_lo(a0 + kLow16 + km_off(kk)), desc_from_lo(b0 + mn_off(kk)), idesc_dv, 1u);
             }
           }
           tc_commit_warp(&bars[Q_EMPTY0 + s]);
           if (!has_next) break;
-          if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[DQ_DRAINED], par, abort_flag, P.status, kStBwdMma)))) break;
-          if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[DO_FULL0 + dsn], dphn, abort_flag, P.status, kStBwdMma)))) break;
-          tc_fence_after();
-          issue_dp(dsn);
+          if constexpr (!SEP_DQ) {
+            if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[DQ_DRAINED], par, abort_flag, P.status, kStBwdMma)))) break;
+            if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[DO_FULL0 + dsn], dphn, abort_flag, P.status, kStBwdMma)))) break;
+            tc_fence_after();
+            issue_dp(dsn);
+          }
           if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[P_READY], par ^ 1, abort_flag, P.status, kStBwdMma)))) break;
           tc_fence_after();
           issue_dv(dsn, false);
@@ -408,40 +414,40 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
       }
     }
     }
-  } else if (DRAIN && warp >= 8) {
+  } else if (warp >= 8) {
     // ------------------------------------------------------------ dQ^T drain (warps 8-11)
-    if constexpr (DRAIN) {
-      reg_inc<kRegsDrain>();
-      // This thread owns head-dim index r of dQ^T; the 128 columns are the tile's queries.  The
-      // whole tile goes to registers and the TMEM columns back to the MMA warp at once; then one
-      // reduction per query: the warp's 32 lanes cover 128 contiguous bytes of that dQ row.
-      const int r = (warp & 3) * 32 + lane;
-      const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
-      const int64_t qrow_base = ((int64_t)bb * p.h + hh) * p.lq;
-      Window win = win0;
-      bool ok = true;
-      int i = first_tile;
-      for (int n = 0; i < P.n_q_tiles; ++n) {
-        if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[DQ_FULL], n & 1, abort_flag, P.status, kStBwdCompute)))) break;
-        tc_fence_after();
-        uint32_t dv[4][32];
+    reg_inc<kRegsDrain>();
+    // This thread owns head-dim index r of dQ^T (head dim 64: of one half of the columns); the
+    // columns are the tile's queries.  The whole tile goes to registers and the TMEM columns back
+    // to the MMA warp at once; then one reduction per query: the warp's 32 lanes cover 128
+    // contiguous bytes of that dQ row.
+    constexpr int COLS = D == 128 ? 128 : 64;
+    const int r = ((warp & 3) * 32 + lane) % D, c0 = D == 128 ? 0 : ((warp & 3) >> 1) * 64;
+    const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
+    const int64_t qrow_base = ((int64_t)bb * p.h + hh) * p.lq;
+    Window win = win0;
+    bool ok = true;
+    int i = first_tile;
+    for (int n = 0; i < P.n_q_tiles; ++n) {
+      if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[DQ_FULL], n & 1, abort_flag, P.status, kStBwdCompute)))) break;
+      tc_fence_after();
+      uint32_t dv[COLS / 32][32];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) tmem_ld32(tmem_dP + lane_off + 32 * j, dv[j]);
-        tc_wait_ld();
-        tc_fence_before();
-        mbar_arrive(&bars[DQ_DRAINED]);
-        const int q_left = p.lq - i * kTileRows;  // a ragged last tile: rows past lq are another head's
-        float* base = p.dq + (qrow_base + (int64_t)i * kTileRows) * 128 + r;
+      for (int j = 0; j < COLS / 32; ++j) tmem_ld32(tmem_dQ + lane_off + c0 + 32 * j, dv[j]);
+      tc_wait_ld();
+      tc_fence_before();
+      mbar_arrive(&bars[DQ_DRAINED]);
+      const int q_left = p.lq - i * kTileRows - c0;  // a ragged last tile: rows past lq are another head's
+      float* base = p.dq + (qrow_base + (int64_t)i * kTileRows + c0) * D + r;
 #pragma unroll
-        for (int c = 0; c < 128; ++c)
-          if (!RAGGED || c < q_left)
-            asm volatile("red.global.add.f32 [%0], %1;" ::"l"(base + c * 128), "f"(__uint_as_float(dv[c >> 5][c & 31])) : "memory");
-        i = next_active(win, i + 1) & kTileIdx;
-      }
+      for (int c = 0; c < COLS; ++c)
+        if (!RAGGED || c < q_left)
+          asm volatile("red.global.add.f32 [%0], %1;" ::"l"(base + c * D), "f"(__uint_as_float(dv[c >> 5][c & 31])) : "memory");
+      i = next_active(win, i + 1) & kTileIdx;
     }
   } else {
     // ------------------------------------------------------------ compute (warps 0-7)
-    if constexpr (DRAIN) reg_inc<kRegsCompute>();
+    reg_inc<kRegsCompute>();
     const int g = warp >> 2;                         // warpgroup: query columns [64g, 64g+64)
     const int r = (warp & 3) * 32 + lane;            // key row of this thread = TMEM lane
     const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
@@ -455,7 +461,6 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
     if (p.mod.kv_pos) kpos = p.mod.kv_pos[mod_row];
     if (p.mod.kv_seg) kseg = p.mod.kv_seg[mod_row];
     if (p.mod.kv_pre) kpre = p.mod.kv_pre[mod_row] != 0;
-    const int64_t qrow_base = ((int64_t)bb * p.h + hh) * p.lq;
     bool ok = true;  // warp-uniform: the tile scan below votes across the warp
     float pf[64];        // P^T of the tile whose dS^T is formed next (this thread's row, 64 columns)
     uint32_t sv[2][32];
@@ -464,7 +469,7 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
     Window& win = win0;
 
     // One loop body serves every tile so that each phase exists once in the instruction
-    // stream: step k does dS^T(k-1), then P^T(k), then the dQ drain of tile k-1.
+    // stream: step k does dS^T(k-1), then P^T(k).
     int i_prev = -1, e_cur = next_active(win, first_tile), i_cur = e_cur & kTileIdx;
     int32_t q0_cur = win.hit_pos0;  // first query position of the tile (used when its positions are contiguous)
     for (int k = 0; ok; ++k) {
@@ -479,12 +484,11 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
         if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[DP_FULL], n & 1, abort_flag, P.status, kStBwdCompute)))) break;
         tc_fence_after();
         tmem_ld32(tmem_dP + lane_off + g * 64, sv[0]);
-        if constexpr (!DRAIN) tmem_ld32(tmem_dP + lane_off + g * 64 + 32, sv[1]);
         tc_wait_ld();
-        // dS^T of the tile before may be overwritten now: dP^T of this tile was issued after the
-        // MMAs that read it (dQ, dK), the tensor pipe runs in issue order, and DP_FULL's commit
-        // covers everything issued before it
-        uint8_t* row_ptr = sdS + g * PANEL_BYTES + r * 128;
+        // this stage of dS^T may be overwritten now: dP^T of this tile was issued after the MMAs that
+        // read what it holds (dQ, dK of DS_ST tiles ago), the tensor pipe runs in issue order, and
+        // DP_FULL's commit covers everything issued before it
+        uint8_t* row_ptr = sdS + (n % DS_ST) * DS_STAGE_BYTES + g * PANEL_BYTES + r * 128;
         const uint64_t scl2 = pack2(p.scale, p.scale);
         // 8 query columns (one 16-byte chunk of this key row of dS^T) from 8 dP^T values
         auto ds_chunk = [&](int ch, const uint32_t* dp) {
@@ -505,21 +509,16 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
           if constexpr (RAGGED)
             *reinterpret_cast<uint4*>(row_ptr + DS_BYTES + ((ch ^ (r & 7)) << 4)) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
         };
-        if constexpr (DRAIN) {
-          // fewer registers per thread here: the second 32 columns are loaded once half of the
-          // first 32 (and the P^T values that went with them) are no longer needed
+        // the second 32 columns are loaded once half of the first 32 (and the P^T values that went
+        // with them) are no longer needed
 #pragma unroll
-          for (int ch = 0; ch < 2; ++ch) ds_chunk(ch, &sv[0][ch * 8]);
-          tmem_ld32(tmem_dP + lane_off + g * 64 + 32, sv[1]);
+        for (int ch = 0; ch < 2; ++ch) ds_chunk(ch, &sv[0][ch * 8]);
+        tmem_ld32(tmem_dP + lane_off + g * 64 + 32, sv[1]);
 #pragma unroll
-          for (int ch = 2; ch < 4; ++ch) ds_chunk(ch, &sv[0][ch * 8]);
-          tc_wait_ld();
+        for (int ch = 2; ch < 4; ++ch) ds_chunk(ch, &sv[0][ch * 8]);
+        tc_wait_ld();
 #pragma unroll
-          for (int ch = 4; ch < 8; ++ch) ds_chunk(ch, &sv[1][(ch - 4) * 8]);
-        } else {
-#pragma unroll
-          for (int ch = 0; ch < 8; ++ch) ds_chunk(ch, &sv[ch >> 2][(ch & 3) * 8]);
-        }
+        for (int ch = 4; ch < 8; ++ch) ds_chunk(ch, &sv[1][(ch - 4) * 8]);
         fence_proxy_async_smem();
         tc_fence_before();
         mbar_arrive(&bars[DS_READY]);
@@ -619,25 +618,6 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
         tc_wait_st();
         tc_fence_before();
         mbar_arrive(&bars[P_READY]);
-      }
-      if constexpr (!DRAIN) {
-        if (have_prev) {
-          // ---- dQ of tile k-1 (head dim 64): rows are queries; add this warpgroup's half of the columns
-          const int n = k - 1;
-          if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[DQ_FULL], n & 1, abort_flag, P.status, kStBwdCompute)))) break;
-          tc_fence_after();
-          constexpr int HALF = D / 2;
-          float* dq_row = p.dq + (qrow_base + (int64_t)i_prev * kTileRows + r) * D + g * HALF;
-          tmem_ld32(tmem_dP + lane_off + g * HALF, sv[0]);
-          tc_wait_ld();
-          const bool q_valid = !RAGGED || i_prev * kTileRows + r < p.lq;
-#pragma unroll
-          for (int e = 0; e < 32; e += 4)
-            if (q_valid) red_add_v4(dq_row + e, __uint_as_float(sv[0][e]), __uint_as_float(sv[0][e + 1]), __uint_as_float(sv[0][e + 2]),
-                       __uint_as_float(sv[0][e + 3]));
-          tc_fence_before();
-          mbar_arrive(&bars[DQ_DRAINED]);
-        }
       }
       if (!have_cur) break;
       i_prev = i_cur;
@@ -741,12 +721,13 @@ __global__ void __launch_bounds__(bwd_threads(D == 128), 1) tc_bwd_kernel(const 
 
 template <int D, bool RAGGED>
 cudaError_t launch_bwd(const BwdTcParams& P, cudaStream_t s) {
-  constexpr size_t kSmem = (4 + bwd_do_stages(D, RAGGED)) * kTileRows * D * 2 + (RAGGED ? 2 : 1) * kTileRows * kTileRows * 2 + 4 * kTileRows * 4 + NUM_BARS * 8 + 64;
+  constexpr size_t kSmem = (4 + bwd_do_stages(D, RAGGED)) * kTileRows * D * 2 +
+                           (D == 64 ? 2 : 1) * (RAGGED ? 2 : 1) * kTileRows * kTileRows * 2 + 4 * kTileRows * 4 + NUM_BARS * 8 + 64;
   constexpr size_t kRequest = kSmem < 120 * 1024 ? 120 * 1024 : kSmem;  // one CTA per SM: it owns all of TMEM
   auto kern = tc_bwd_kernel<D, RAGGED>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRequest);
   if (e != cudaSuccess) return e;
-  kern<<<P.n_kv_tiles * P.p.b * P.p.h, bwd_threads(D == 128), kRequest, s>>>(P);
+  kern<<<P.n_kv_tiles * P.p.b * P.p.h, kBwdThreads, kRequest, s>>>(P);
   count_launch();
   return cudaGetLastError();
 }
