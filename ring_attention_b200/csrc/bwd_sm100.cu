@@ -812,8 +812,7 @@ cudaError_t tc_bwd_block(const BwdParams& p, cudaStream_t s) {
     }
     TileMeta* mq = meta;
     TileMeta* mk = meta + (size_t)p.b * P.n_q_tiles;
-    if ((e = launch_tile_meta(mq, p.mod.q_pos, p.mod.q_seg, p.mod.q_pre, p.b, p.lq, s)) == cudaSuccess)
-      e = launch_tile_meta(mk, p.mod.kv_pos, p.mod.kv_seg, p.mod.kv_pre, p.b, p.lk, s);
+    e = launch_tile_meta(mq, mk, p.mod, p.b, p.lq, p.lk, s);
     P.meta_q = mq;
     P.meta_kv = mk;
   }

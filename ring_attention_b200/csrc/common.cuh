@@ -83,10 +83,15 @@ cudaError_t simt_wide_bwd(const BwdParams& p, int dtype, cudaStream_t s);
 cudaError_t launch_finalize(int b, int h, int lq, int dv, const float* o, const float* m, const float* l,
                             const float* o2, const float* m2, const float* l2, TensorView out, int dtype,
                             float* lse, cudaStream_t s);
-cudaError_t launch_delta(int b, int h, int lq, int dv, TensorView out, TensorView dout, int dtype,
-                         float* delta, cudaStream_t s);
+// delta = rowsum(out * dout); with nl2 also the row terms below (clamped, padded to `pitch` >= lq rows per
+// (batch, head)); with dq also clears its [b, h, lq, dk] floats (16-byte aligned when dk is a multiple of 4).
+cudaError_t launch_bwd_rows(int b, int h, int lq, int pitch, int dk, int dv, TensorView out, TensorView dout, int dtype,
+                            const float* lse, float scale, float* delta, float* nl2, float* nds, float* dq, cudaStream_t s);
 cudaError_t launch_cast_from_f32(int b, int h, int len, int d, const float* src, TensorView dst,
                                  int dtype, cudaStream_t s);
+// The three gradients of a backward, one launch.
+cudaError_t launch_cast_grads(int b, int h, int lq, int lk, int dk, int dv, const float* dq, TensorView dq_out, const float* dkk,
+                              TensorView dk_out, const float* dvv, TensorView dv_out, int dtype, cudaStream_t s);
 // nl2 = min(-lse * log2(e), 1e30) (clamp left out when !clamp), nds = -delta * scale, for bh runs of lq rows;
 // the results have `pitch` >= lq rows per run, of which the last pitch - lq are padding.
 cudaError_t launch_bwd_row_terms(const float* lse, const float* delta, float scale, int clamp, int64_t bh, int lq,

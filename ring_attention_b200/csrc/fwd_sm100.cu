@@ -477,8 +477,24 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
 }
 
 // -----------------------------------------------------------------------------------------
-__global__ void tile_meta_kernel(TileMeta* __restrict__ out, const int32_t* __restrict__ pos,
-                                 const int32_t* __restrict__ seg, const uint8_t* __restrict__ pre, int len) {
+// Both sides of a block in one launch (blockIdx.z: queries, keys).
+struct MetaSide {
+  TileMeta* out;  // [b][n_tiles]
+  const int32_t *pos, *seg;
+  const uint8_t* pre;
+  int len;
+};
+struct MetaSides {
+  MetaSide side[2];
+};
+
+__global__ void tile_meta_kernel(const MetaSides sides) {
+  const MetaSide& sd = sides.side[blockIdx.z];
+  TileMeta* __restrict__ out = sd.out;
+  const int32_t* __restrict__ pos = sd.pos;
+  const int32_t* __restrict__ seg = sd.seg;
+  const uint8_t* __restrict__ pre = sd.pre;
+  const int len = sd.len;
   // one warp per tile: 4 tokens per lane; a ragged last tile is summarised over the tokens it has
   const int n_tiles = tiles_of(len);
   const int tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -633,11 +649,11 @@ bool make_tile_map(CUtensorMap* map, const TensorView& t, int b, int len, int h,
   return true;
 }
 
-cudaError_t launch_tile_meta(TileMeta* out, const int32_t* pos, const int32_t* seg, const uint8_t* pre, int b,
-                             int len, cudaStream_t s) {
-  const int n_tiles = tiles_of(len);
-  dim3 grid((n_tiles + 7) / 8, b);
-  tile_meta_kernel<<<grid, 256, 0, s>>>(out, pos, seg, pre, len);
+cudaError_t launch_tile_meta(TileMeta* out_q, TileMeta* out_kv, const ModParams& m, int b, int lq, int lk, cudaStream_t s) {
+  const MetaSides sides = {{{out_q, m.q_pos, m.q_seg, m.q_pre, lq}, {out_kv, m.kv_pos, m.kv_seg, m.kv_pre, lk}}};
+  const int n_tiles = tiles_of(lq > lk ? lq : lk);
+  dim3 grid((n_tiles + 7) / 8, b, 2);
+  tile_meta_kernel<<<grid, 256, 0, s>>>(sides);
   count_launch();
   return cudaGetLastError();
 }
@@ -691,8 +707,7 @@ cudaError_t tc_fwd_block(const FwdParams& p, cudaStream_t s) {
     if ((e = scratch_alloc((void**)&meta, n * sizeof(TileMeta), s)) != cudaSuccess) return e;
     TileMeta* mq = meta;
     TileMeta* mk = meta + (size_t)p.b * P.n_q_tiles;
-    if ((e = launch_tile_meta(mq, p.mod.q_pos, p.mod.q_seg, p.mod.q_pre, p.b, p.lq, s)) == cudaSuccess)
-      e = launch_tile_meta(mk, p.mod.kv_pos, p.mod.kv_seg, p.mod.kv_pre, p.b, p.lk, s);
+    e = launch_tile_meta(mq, mk, p.mod, p.b, p.lq, p.lk, s);
     P.meta_q = mq;
     P.meta_kv = mk;
   }
@@ -720,7 +735,7 @@ cudaError_t tc_fwd_block(const FwdParams& p, cudaStream_t s) {
 // exits, and nothing is allocated or freed by a call.
 //
 // All calls share the one array and it keeps whatever the last call wrote.  The summaries
-// a call needs are completely rewritten by that call's own first two launches, so nothing
+// a call needs are completely rewritten by that call's own first launch, so nothing
 // has to be cleared; but two calls that overlap on the GPU (different streams, or two host
 // threads) overwrite each other's summaries.  Callers must serialise them.
 // -----------------------------------------------------------------------------------------
@@ -809,8 +824,7 @@ extern "C" int ra_fwd_block_static(const ra_shape_t* shape, const ra_tensor_t* q
     if ((e = static_tile_meta(&meta)) != cudaSuccess) return fail_cuda(e, "cudaGetSymbolAddress(static scratch)");
     TileMeta* mq = meta;
     TileMeta* mk = meta + (size_t)p.b * P.n_q_tiles;
-    if ((e = launch_tile_meta(mq, p.mod.q_pos, p.mod.q_seg, p.mod.q_pre, p.b, p.lq, s)) != cudaSuccess ||
-        (e = launch_tile_meta(mk, p.mod.kv_pos, p.mod.kv_seg, p.mod.kv_pre, p.b, p.lk, s)) != cudaSuccess)
+    if ((e = launch_tile_meta(mq, mk, p.mod, p.b, p.lq, p.lk, s)) != cudaSuccess)
       return fail_cuda(e, "tile summaries");
     P.meta_q = mq;
     P.meta_kv = mk;

@@ -223,8 +223,8 @@ int ra_bwd_delta(const ra_shape_t* shape, const ra_tensor_t* out, const ra_tenso
   if ((rc = check_shape(shape))) return rc;
   if ((rc = check_tensor(out, "out")) || (rc = check_tensor(dout, "dout"))) return rc;
   if (!delta) return fail(-6, "delta is NULL");
-  cudaError_t e = launch_delta(shape->b, shape->h, shape->lq, shape->dv, view(out), view(dout),
-                               shape->dtype, delta, (cudaStream_t)stream);
+  cudaError_t e = launch_bwd_rows(shape->b, shape->h, shape->lq, shape->lq, shape->dk, shape->dv, view(out), view(dout),
+                                  shape->dtype, nullptr, 0.f, delta, nullptr, nullptr, nullptr, (cudaStream_t)stream);
   if (e != cudaSuccess) return fail_cuda(e, "delta");
   return 0;
 }

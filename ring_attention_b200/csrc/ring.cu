@@ -1336,13 +1336,14 @@ int ra_ring_bwd(ra_ring_t* ring, const ra_shape_t* shape, const ra_tensor_t* q,
     return fail(-39, "the plan was made for a ring of %d ranks", ring->plan->nranks);
   if ((rc = begin_call(ring, 1, stream))) return rc;
 
-  cudaError_t e = launch_delta(shape->b, shape->h, shape->lq, shape->dv, tv(out), p.dout,
-                               shape->dtype, delta, stream);
-  if (e != cudaSuccess) return fail_cuda(e, "delta");
+  // delta, the row terms (once per backward, not once per block launch) and a cleared dQ accumulator
+  const bool terms = current_impl() != RA_IMPL_SIMT;
+  cudaError_t e = launch_bwd_rows(shape->b, shape->h, shape->lq, row_pitch(shape->lq), shape->dk, shape->dv, tv(out), p.dout,
+                                  shape->dtype, lse, shape->sm_scale, delta, terms ? row_nl2 : nullptr,
+                                  terms ? row_nds : nullptr, dq_acc, stream);
+  if (e != cudaSuccess) return fail_cuda(e, "row terms");
   p.delta = delta;
-  if (current_impl() != RA_IMPL_SIMT) {  // once per backward, not once per block launch
-    e = launch_bwd_row_terms(lse, delta, shape->sm_scale, 1, (int64_t)shape->b * shape->h, shape->lq, row_pitch(shape->lq), row_nl2, row_nds, stream);
-    if (e != cudaSuccess) return fail_cuda(e, "row terms");
+  if (terms) {
     p.row_nl2 = row_nl2;
     p.row_nds = row_nds;
   }
@@ -1360,8 +1361,10 @@ int ra_ring_bwd(ra_ring_t* ring, const ra_shape_t* shape, const ra_tensor_t* q,
              (current_impl() == RA_IMPL_AUTO && tc_bwd_ragged_unsupported_reason(p, shape->dtype) == nullptr);
     if (!direct) p.dk_out = p.dv_out = TensorView{nullptr, 0, 0, 0};
   }
-  RA_CUDA(cudaMemsetAsync(dq_acc, 0, direct ? dq_b : dq_b + dk_b + dv_b, stream), "cudaMemsetAsync");
-  count_launch();
+  if (!direct) {
+    RA_CUDA(cudaMemsetAsync(dk_acc, 0, dk_b + dv_b, stream), "cudaMemsetAsync");
+    count_launch();
+  }
   if (direct) {
     if ((rc = block_mark(ring, 1, stream))) return rc;
     e = tc_bwd_block(p, stream);
@@ -1543,9 +1546,8 @@ int ra_ring_bwd(ra_ring_t* ring, const ra_shape_t* shape, const ra_tensor_t* q,
         (e = launch_add_f32(dv_acc + off * shape->dv, own2_dv, (int64_t)rows2 * shape->dv, stream)) != cudaSuccess)
       return fail_cuda(e, "add");
   }
-  if ((e = launch_cast_from_f32(shape->b, shape->h, shape->lq, shape->dk, dq_acc, tv(dq), shape->dtype, stream)) != cudaSuccess ||
-      (e = launch_cast_from_f32(shape->b, shape->h, shape->lk, shape->dk, dk_acc, tv(dk), shape->dtype, stream)) != cudaSuccess ||
-      (e = launch_cast_from_f32(shape->b, shape->h, shape->lk, shape->dv, dv_acc, tv(dv), shape->dtype, stream)) != cudaSuccess)
+  if ((e = launch_cast_grads(shape->b, shape->h, shape->lq, shape->lk, shape->dk, shape->dv, dq_acc, tv(dq), dk_acc, tv(dk), dv_acc,
+                             tv(dv), shape->dtype, stream)) != cudaSuccess)
     return fail_cuda(e, "cast");
   return end_call(ring, 1, stream);
 }

@@ -461,38 +461,149 @@ __global__ void finalize_kernel(int b, int h, int lq, int dv, const float* __res
   }
 }
 
-// delta = rowsum(out * dout) (ring_kernel.py:387-409; ring.py:151).  One warp per row.
+// 16 bytes of T as floats.
 template <typename T>
-__global__ void delta_kernel(int b, int h, int lq, int dv, TensorView out, TensorView dout,
-                             float* __restrict__ delta) {
-  int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  int lane = threadIdx.x & 31;
-  int64_t nrows = (int64_t)b * h * lq;
-  if (row >= nrows) return;
-  int r = (int)(row % lq);
-  int hh = (int)((row / lq) % h);
-  int bb = (int)(row / ((int64_t)lq * h));
-  const T* a = (const T*)out.ptr + (int64_t)bb * out.sb + (int64_t)r * out.sl + (int64_t)hh * out.sh;
-  const T* g = (const T*)dout.ptr + (int64_t)bb * dout.sb + (int64_t)r * dout.sl + (int64_t)hh * dout.sh;
-  float acc = 0.f;
-  for (int c = lane; c < dv; c += 32) acc = fmaf(load_as_float(a + c), load_as_float(g + c), acc);
+struct Vec16;
+template <>
+struct Vec16<float> {
+  static constexpr int N = 4;
+  static __device__ __forceinline__ void load(const float* p, float (&x)[4]) {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    x[0] = v.x, x[1] = v.y, x[2] = v.z, x[3] = v.w;
+  }
+  static __device__ __forceinline__ void store(float* p, const float (&x)[4]) {
+    *reinterpret_cast<float4*>(p) = make_float4(x[0], x[1], x[2], x[3]);
+  }
+};
+template <>
+struct Vec16<__nv_bfloat16> {
+  static constexpr int N = 8;
+  static __device__ __forceinline__ void load(const __nv_bfloat16* p, float (&x)[8]) {
+    const uint4 v = *reinterpret_cast<const uint4*>(p);
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (lane == 0) delta[row] = acc;
+    for (int i = 0; i < 4; ++i) {
+      x[2 * i] = __uint_as_float(w[i] << 16);
+      x[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+    }
+  }
+  static __device__ __forceinline__ void store(__nv_bfloat16* p, const float (&x)[8]) {
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const __nv_bfloat162 h = __floats2bfloat162_rn(x[2 * i], x[2 * i + 1]);
+      w[i] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+    *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+};
+
+// Whether every row of `dim` elements of a strided tensor starts and ends on 16 bytes.
+template <typename T>
+static bool rows_of_16_bytes(const TensorView& t, int dim) {
+  constexpr int N = 16 / sizeof(T);
+  return (reinterpret_cast<uintptr_t>(t.ptr) & 15) == 0 && t.sb % N == 0 && t.sl % N == 0 && t.sh % N == 0 && dim % N == 0;
 }
 
-template <typename T>
-__global__ void cast_kernel(int b, int h, int len, int d, const float* __restrict__ src,
-                            TensorView dst) {
-  int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  int lane = threadIdx.x & 31;
-  int64_t nrows = (int64_t)b * h * len;
-  if (row >= nrows) return;
-  int r = (int)(row % len);
-  int hh = (int)((row / len) % h);
-  int bb = (int)(row / ((int64_t)len * h));
-  T* out = (T*)dst.ptr + (int64_t)bb * dst.sb + (int64_t)r * dst.sl + (int64_t)hh * dst.sh;
-  for (int c = lane; c < d; c += 32) store_from_float(out + c, src[row * d + c]);
+// What the backward needs of every query row before its block kernels: delta = rowsum(out * dout)
+// (ring_kernel.py:387-409; ring.py:151), the two row terms (`row_terms` below) if nl2 is set, and a
+// cleared dQ row if dq is set.  Sixteen lanes per row, 16-byte accesses when VEC.  One pass where
+// two kernels and a clear stood: bound by memory, 8k tokens of 32 heads (d 128) take it 52 us and took
+// them 89 (41 at the copy rate).
+__device__ __forceinline__ void row_terms(float L, float delta, float scale, int clamp, float* nl2, float* nds) {
+  const float x = -L * 1.4426950408889634f;
+  *nl2 = clamp ? fminf(x, 1e30f) : x;
+  // a row that saw no key has delta = NaN; without a dense bias it contributes nothing
+  *nds = (clamp && L == -INFINITY) ? 0.f : -delta * scale;
+}
+
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(256) bwd_rows_kernel(int64_t nrows, int h, int lq, int pitch, int dk, int dv, TensorView out,
+                                                       TensorView dout, const float* __restrict__ lse, float scale,
+                                                       float* __restrict__ delta, float* __restrict__ nl2,
+                                                       float* __restrict__ nds, float* __restrict__ dq) {
+  const int64_t prow = (int64_t)blockIdx.x * 16 + (threadIdx.x >> 4);  // row of the padded [b, h, pitch] terms
+  const int lane = threadIdx.x & 15;
+  const int64_t bh = prow / pitch;
+  const int r = (int)(prow - bh * pitch);
+  const bool in = prow < nrows && r < lq;
+  float acc = 0.f;
+  const int64_t row = bh * lq + r;
+  if (in) {
+    const int hh = (int)(bh % h), bb = (int)(bh / h);
+    const T* a = (const T*)out.ptr + (int64_t)bb * out.sb + (int64_t)r * out.sl + (int64_t)hh * out.sh;
+    const T* g = (const T*)dout.ptr + (int64_t)bb * dout.sb + (int64_t)r * dout.sl + (int64_t)hh * dout.sh;
+    if constexpr (VEC) {
+      constexpr int N = Vec16<T>::N;
+      for (int c = lane * N; c < dv; c += 16 * N) {
+        float x[N], y[N];
+        Vec16<T>::load(a + c, x);
+        Vec16<T>::load(g + c, y);
+#pragma unroll
+        for (int e = 0; e < N; ++e) acc = fmaf(x[e], y[e], acc);
+      }
+    } else {
+      for (int c = lane; c < dv; c += 16) acc = fmaf(load_as_float(a + c), load_as_float(g + c), acc);
+    }
+    if (dq) {
+      float* q = dq + row * dk;
+      if (dk % 4 == 0) {
+        for (int c = lane * 4; c < dk; c += 64) *reinterpret_cast<float4*>(q + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+      } else {
+        for (int c = lane; c < dk; c += 16) q[c] = 0.f;
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (lane == 0 && prow < nrows) {
+    if (in) delta[row] = acc;
+    if (nl2) {
+      if (in) {
+        row_terms(lse[row], acc, scale, 1, nl2 + prow, nds + prow);
+      } else {  // padding: P = 0 and dS = 0
+        nl2[prow] = -1e30f;
+        nds[prow] = 0.f;
+      }
+    }
+  }
+}
+
+// fp32 [b, h, len, d] rows -> T at any strides; up to three tensors in one launch (blockIdx.y).  VEC: one
+// 16-byte store per thread, else one element.  The dQ of 8k tokens of 32 heads (d 128): 55 -> 33 us.
+struct CastJob {
+  const float* src;
+  TensorView dst;
+  int len, d;
+};
+struct CastJobs {
+  CastJob job[3];
+};
+
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(256) cast_kernel(const CastJobs jobs, int b, int h) {
+  constexpr int N = VEC ? Vec16<T>::N : 1;
+  const CastJob& j = jobs.job[blockIdx.y];
+  const int per_row = j.d / N;
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t row = i / per_row;
+  if (row >= (int64_t)b * h * j.len) return;
+  const int c = (int)(i - row * per_row) * N;
+  const int64_t bh = row / j.len;
+  const int r = (int)(row - bh * j.len), hh = (int)(bh % h), bb = (int)(bh / h);
+  T* out = (T*)j.dst.ptr + (int64_t)bb * j.dst.sb + (int64_t)r * j.dst.sl + (int64_t)hh * j.dst.sh + c;
+  const float* src = j.src + row * j.d + c;
+  if constexpr (VEC) {
+    float x[N];
+#pragma unroll
+    for (int e = 0; e < N; e += 4) {
+      const float4 v = *reinterpret_cast<const float4*>(src + e);
+      x[e] = v.x, x[e + 1] = v.y, x[e + 2] = v.z, x[e + 3] = v.w;
+    }
+    Vec16<T>::store(out, x);
+  } else {
+    store_from_float(out, *src);
+  }
 }
 
 __global__ void add_f32_kernel(float* __restrict__ dst, const float* __restrict__ src, int64_t n) {
@@ -594,28 +705,59 @@ cudaError_t launch_finalize(int b, int h, int lq, int dv, const float* o, const 
   return cudaGetLastError();
 }
 
-cudaError_t launch_delta(int b, int h, int lq, int dv, TensorView out, TensorView dout, int dtype,
-                         float* delta, cudaStream_t s) {
-  int64_t rows = (int64_t)b * h * lq;
-  int grid = (int)((rows + 7) / 8);
-  if (dtype == RA_DTYPE_F32)
-    delta_kernel<float><<<grid, 256, 0, s>>>(b, h, lq, dv, out, dout, delta);
+template <typename T>
+static cudaError_t launch_bwd_rows_t(int b, int h, int lq, int pitch, int dk, int dv, TensorView out, TensorView dout,
+                                     const float* lse, float scale, float* delta, float* nl2, float* nds, float* dq,
+                                     cudaStream_t s) {
+  const int64_t rows = (int64_t)b * h * pitch;
+  const unsigned grid = (unsigned)((rows + 15) / 16);
+  if (rows_of_16_bytes<T>(out, dv) && rows_of_16_bytes<T>(dout, dv))
+    bwd_rows_kernel<T, true><<<grid, 256, 0, s>>>(rows, h, lq, pitch, dk, dv, out, dout, lse, scale, delta, nl2, nds, dq);
   else
-    delta_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(b, h, lq, dv, out, dout, delta);
+    bwd_rows_kernel<T, false><<<grid, 256, 0, s>>>(rows, h, lq, pitch, dk, dv, out, dout, lse, scale, delta, nl2, nds, dq);
   count_launch();
   return cudaGetLastError();
 }
 
-cudaError_t launch_cast_from_f32(int b, int h, int len, int d, const float* src, TensorView dst,
-                                 int dtype, cudaStream_t s) {
-  int64_t rows = (int64_t)b * h * len;
-  int grid = (int)((rows + 7) / 8);
-  if (dtype == RA_DTYPE_F32)
-    cast_kernel<float><<<grid, 256, 0, s>>>(b, h, len, d, src, dst);
+cudaError_t launch_bwd_rows(int b, int h, int lq, int pitch, int dk, int dv, TensorView out, TensorView dout, int dtype,
+                            const float* lse, float scale, float* delta, float* nl2, float* nds, float* dq, cudaStream_t s) {
+  return dtype == RA_DTYPE_F32
+             ? launch_bwd_rows_t<float>(b, h, lq, pitch, dk, dv, out, dout, lse, scale, delta, nl2, nds, dq, s)
+             : launch_bwd_rows_t<__nv_bfloat16>(b, h, lq, pitch, dk, dv, out, dout, lse, scale, delta, nl2, nds, dq, s);
+}
+
+template <typename T>
+static cudaError_t launch_cast_t(const CastJobs& jobs, int n, int b, int h, cudaStream_t s) {
+  bool vec = true;
+  for (int i = 0; i < n; ++i)
+    vec = vec && rows_of_16_bytes<T>(jobs.job[i].dst, jobs.job[i].d) && (reinterpret_cast<uintptr_t>(jobs.job[i].src) & 15) == 0;
+  int64_t most = 0;
+  for (int i = 0; i < n; ++i) {
+    const int64_t threads = (int64_t)b * h * jobs.job[i].len * (vec ? jobs.job[i].d / Vec16<T>::N : jobs.job[i].d);
+    most = threads > most ? threads : most;
+  }
+  const dim3 grid((unsigned)((most + 255) / 256), n);
+  if (vec)
+    cast_kernel<T, true><<<grid, 256, 0, s>>>(jobs, b, h);
   else
-    cast_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(b, h, len, d, src, dst);
+    cast_kernel<T, false><<<grid, 256, 0, s>>>(jobs, b, h);
   count_launch();
   return cudaGetLastError();
+}
+
+cudaError_t launch_cast_from_f32(int b, int h, int len, int d, const float* src, TensorView dst, int dtype, cudaStream_t s) {
+  CastJobs jobs = {};
+  jobs.job[0] = {src, dst, len, d};
+  return dtype == RA_DTYPE_F32 ? launch_cast_t<float>(jobs, 1, b, h, s) : launch_cast_t<__nv_bfloat16>(jobs, 1, b, h, s);
+}
+
+cudaError_t launch_cast_grads(int b, int h, int lq, int lk, int dk, int dv, const float* dq, TensorView dq_out, const float* dkk,
+                              TensorView dk_out, const float* dvv, TensorView dv_out, int dtype, cudaStream_t s) {
+  CastJobs jobs = {};
+  jobs.job[0] = {dq, dq_out, lq, dk};
+  jobs.job[1] = {dkk, dk_out, lk, dk};
+  jobs.job[2] = {dvv, dv_out, lk, dv};
+  return dtype == RA_DTYPE_F32 ? launch_cast_t<float>(jobs, 3, b, h, s) : launch_cast_t<__nv_bfloat16>(jobs, 3, b, h, s);
 }
 
 cudaError_t launch_strict_nan(int b, int h, int lq, int lk, int dk_dim, int dv_dim, const float* lse, float* dq,
@@ -638,10 +780,7 @@ __global__ void bwd_row_terms_kernel(const float* __restrict__ lse, const float*
     nds[i] = 0.f;
     return;
   }
-  const float L = lse[bh * lq + r], x = -L * 1.4426950408889634f;
-  nl2[i] = clamp ? fminf(x, 1e30f) : x;
-  // a row that saw no key has delta = NaN; without a dense bias it contributes nothing
-  nds[i] = (clamp && L == -INFINITY) ? 0.f : -delta[bh * lq + r] * scale;
+  row_terms(lse[bh * lq + r], delta[bh * lq + r], scale, clamp, nl2 + i, nds + i);
 }
 
 __global__ void add_rows_f32_kernel(float* __restrict__ dst, const float* __restrict__ src, int64_t seg_elems,

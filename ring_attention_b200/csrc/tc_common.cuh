@@ -183,9 +183,8 @@ __device__ __noinline__ void bias_scores_tmem(uint32_t taddr, int ncols, bool al
 bool make_tile_map(CUtensorMap* map, const TensorView& t, int b, int len, int h, int d, int box_rows,
                    const char** why);
 
-// Launches the kernel that fills TileMeta[b][n_tiles] for one side (q or kv).
-cudaError_t launch_tile_meta(TileMeta* out, const int32_t* pos, const int32_t* seg, const uint8_t* pre,
-                             int b, int len, cudaStream_t s);
+// Launches the kernel that fills TileMeta[b][n_tiles] for the query side and the key side.
+cudaError_t launch_tile_meta(TileMeta* out_q, TileMeta* out_kv, const ModParams& m, int b, int lq, int lk, cudaStream_t s);
 
 // Stream-ordered scratch (tile summaries) from a memory pool of this library, one per device,
 // that keeps what it has been given: the default pool hands unused memory back to the driver at
