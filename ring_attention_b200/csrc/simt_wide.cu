@@ -4,13 +4,12 @@
 // 4 x 4 patch per thread fed by eight 4-byte loads per 16 FMAs, both operands staged again for
 // every 32 columns of the head dim, and the mask evaluated per pair on every tile, seen or not.
 // Here whole operand tiles are staged once by asynchronous copies, a thread owns R x 4 scores and
-// reads its operands as 16-byte vectors (R = 8: 16 shared-memory wavefronts per 128 FMA
-// instructions, half of what that pipe can take in the time), products run on packed fp32 pairs,
+// reads its operands as 16-byte vectors in products on packed fp32 pairs,
 // and tiles are classified from position / segment ranges, so that only tiles which really mix
 // visible and masked pairs look at pairs.
 // Measured (device time of the whole pass, before -> now): 2048 x 2048, b 2, h 4, d 64, no mask:
-// forward 529 -> 337 us, backward 1125 -> 722 us; d 128: 933 -> 601, 2977 -> 1286 us; causal 1024,
-// b 1, h 4, d 64: 228 -> 91, 423 -> 129 us.  What bounds it now is the FMA pipe together with the
+// forward 529 -> 320 us, backward 1125 -> 710 us; d 128: 933 -> 601, 2977 -> 1283 us; causal 1024,
+// b 1, h 4, d 64: 228 -> 83, 423 -> 105 us.  What bounds it now is the FMA pipe together with the
 // shared-memory reads (25 to 33 of 74 TFLOP/s): one or two warps per scheduler do not hide them all.
 #include <math.h>
 
@@ -269,7 +268,7 @@ __device__ __forceinline__ void score_patch(float (&s)[R][4], const uint64_t (&a
 // QK^T, K of the next tile under the softmax and PV.
 // ---------------------------------------------------------------------------------------
 template <typename T, int D_PAD, int R, int TY>
-__global__ void __launch_bounds__(16 * TY) wide_fwd_kernel(const FwdParams p) {
+__global__ void __launch_bounds__(16 * TY, D_PAD == 64 ? 2 : 1) wide_fwd_kernel(const FwdParams p) {
   constexpr int P = D_PAD + 4, BM = R * TY, NT = 16 * TY, NO = D_PAD / 32;
   extern __shared__ __align__(16) float smem[];
   float* Qs = smem;
@@ -435,7 +434,7 @@ __device__ __forceinline__ void add_rows(float* base, const uint64_t (&v)[R][D_P
 // dQ always is).  The next Q and dO tiles arrive under the dQ product.
 // ---------------------------------------------------------------------------------------
 template <typename T, int D_PAD, int TY>
-__global__ void __launch_bounds__(16 * TY) wide_bwd_kernel(const BwdParams p, int splits) {
+__global__ void __launch_bounds__(16 * TY, D_PAD == 64 ? 2 : 1) wide_bwd_kernel(const BwdParams p, int splits) {
   constexpr int P = D_PAD + 4, R = BT / TY, NT = 16 * TY, NO = D_PAD / 32;
   extern __shared__ __align__(16) float smem[];
   float* Qs = smem;
@@ -578,15 +577,21 @@ cudaError_t launch_bwd(const BwdParams& p, cudaStream_t s) {
 
 template <typename T>
 cudaError_t dispatch_fwd(const FwdParams& p, cudaStream_t s) {
-  // 64 query rows per CTA when that fills the chip, 32 otherwise
+  // 64 query rows per CTA when that fills the chip, 32 otherwise; 256 threads, since more warps hide
+  // more of the shared-memory latency than larger patches save (2048 x 2048: 337 -> 320 us, causal 1k:
+  // 91 -> 83 us against 128 threads)
   const bool small = (int64_t)((p.lq + 63) / 64) * p.h * p.b < 148;
-  if (max(p.dk, p.dv) <= 64) return small ? launch_fwd<T, 64, 4, 8>(p, s) : launch_fwd<T, 64, 8, 8>(p, s);
-  return small ? launch_fwd<T, 128, 4, 8>(p, s) : launch_fwd<T, 128, 4, 16>(p, s);
+  if (max(p.dk, p.dv) <= 64) return small ? launch_fwd<T, 64, 2, 16>(p, s) : launch_fwd<T, 64, 4, 16>(p, s);
+  return small ? launch_fwd<T, 128, 2, 16>(p, s) : launch_fwd<T, 128, 4, 16>(p, s);
 }
 
 template <typename T>
 cudaError_t dispatch_bwd(const BwdParams& p, cudaStream_t s) {
-  return max(p.dk_dim, p.dv_dim) <= 64 ? launch_bwd<T, 64, 8>(p, s) : launch_bwd<T, 128, 16>(p, s);
+  if (max(p.dk_dim, p.dv_dim) > 64) return launch_bwd<T, 128, 16>(p, s);
+  // few key tiles: 256 threads shorten a CTA's chain (causal 1k: 117 -> 105 us); many: 128 threads read
+  // less shared memory per FMA (2048 x 2048: 710 us against 755)
+  const bool small = (int64_t)((p.lk + BT - 1) / BT) * p.h * p.b < 148;
+  return small ? launch_bwd<T, 64, 16>(p, s) : launch_bwd<T, 64, 8>(p, s);
 }
 
 }  // namespace
