@@ -195,13 +195,16 @@ def _dense_mod(bias: Optional[torch.Tensor], b: int, h: int, lq: int, lk: int):
         bias = bias[:, None]
     if bias.shape[0] != b or bias.shape[1] not in (1, h) or bias.shape[2] != lq or bias.shape[3] != lk:
         raise ValueError(f"bias shape {tuple(bias.shape)} does not match [b={b}, h={h} or 1, {lq}, {lk}]")
-    bias = bias.contiguous()
+    # The kernels read any batch, head and row strides (0 for a broadcast axis).  A view is copied only
+    # where its rows are not consecutive floats on 16-byte boundaries.
+    strides = [0 if bias.shape[i] == 1 else bias.stride(i) for i in range(3)]
+    if (bias.stride(3) != 1 and lk > 1) or bias.data_ptr() % 16 or any(s % 4 for s in strides):
+        bias = bias.contiguous()
+        strides = [0 if bias.shape[i] == 1 else bias.stride(i) for i in range(3)]
     m = RaScoreMod()
     m.kinds = _lib.RA_MOD_DENSE
     m.bias = bias.data_ptr()
-    m.bias_stride_b = bias.stride(0)
-    m.bias_stride_h = 0 if bias.shape[1] == 1 else bias.stride(1)
-    m.bias_stride_q = bias.stride(2)
+    m.bias_stride_b, m.bias_stride_h, m.bias_stride_q = strides
     return m, bias
 
 
@@ -356,8 +359,9 @@ def _host_bwd(ring, q, k, v, out, lse, do, sm_scale, bias_fn, q_kwargs, kv_kwarg
                                C.byref(mod), _ptr(L), _ptr(delta), C.byref(_view_blhd(doc)), _ptr(dq), _ptr(dkk),
                                _ptr(dvv), _stream()))
         del keep
-        qc, dq, doc, L, delta = _rotate(ring, [qc, dq, doc, L, delta])  # ring.py:195
-        qk = _rotate_kwargs(ring, qk)
+        if ring.size > 1:  # a ring of one has everything at home
+            qc, dq, doc, L, delta = _rotate(ring, [qc, dq, doc, L, delta])  # ring.py:195
+            qk = _rotate_kwargs(ring, qk)
 
     def cast(acc, like, n):
         dst = torch.empty_like(like)
