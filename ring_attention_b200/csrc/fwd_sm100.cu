@@ -323,18 +323,18 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
 #pragma unroll
       for (int c = 0; c < 4; ++c) tmem_ld32(tmem_S[t] + lane_off + c * 32, r[c]);
       tc_wait_ld();
-      // sc: what is left to multiply the register values by (the ALiBi form has the scale in already)
-      float sc = scale2;
+      // ALiBi: scale * s - slope * (q_pos - kv_pos) with kv_pos = k0 + column (ring_test.py-style
+      // callables).  The column's part goes on the raw scores, divided by the scale; the row's part
+      // (position differences are exact in fp32) joins the running max: one FMA per score
+      // (64k windowed tokens, d 64: 7.63 -> 7.07 ms against two per score)
+      float row_bias = 0.f;
       if (alibi_inline) {
-        // scale * s - slope * (q_pos - kv_pos), times log2(e): the bias of ring_test.py-style ALiBi
-        // callables, with kv_pos = k0 + column; the differences are exact in fp32
-        const float r_i = slope2 * (float)(k0 - qpos);
+        row_bias = slope2 * (float)(k0 - qpos);
 #pragma unroll
         for (int c = 0; c < 4; ++c)
 #pragma unroll
           for (int e = 0; e < 32; ++e)
-            r[c][e] = __float_as_uint(fmaf(slope2, (float)(c * 32 + e), fmaf(__uint_as_float(r[c][e]), scale2, r_i)));
-        sc = 1.f;
+            r[c][e] = __float_as_uint(fmaf(alibi_over_scale, (float)(c * 32 + e), __uint_as_float(r[c][e])));
       }
       if (need_mask) {
 #pragma unroll
@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
 #pragma unroll
         for (int e = 0; e < 32; e += 2) mxa[c] = max3(mxa[c], __uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1]));
       const float mx = fmaxf(fmaxf(mxa[0], mxa[1]), fmaxf(mxa[2], mxa[3]));
-      const float m_new = fmaxf(m_true, mx * sc);
+      const float m_new = fmaxf(m_true, fmaf(mx, scale2, row_bias));
       m_true = m_new;
       const bool need = (m_new > m_ref + kRescaleThreshold) || (m_ref == -INFINITY && m_new != -INFINITY);
       if (__any_sync(0xffffffffu, need)) {
@@ -371,11 +371,11 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
           }
         }
       }
-      const float neg_m = (m_ref == -INFINITY) ? 0.f : -m_ref;
-      // p = 2^(s * sc - m) on pairs of columns: the first kPolyPairs of every 16 pairs take the
+      const float neg_m = (m_ref == -INFINITY) ? 0.f : row_bias - m_ref;
+      // p = 2^(s * scale2 + row_bias - m) on pairs of columns: the first kPolyPairs of every 16 pairs take the
       // polynomial on the FMA pipe, the rest the special-function unit, so that the two pipes
       // finish together; one packed sum per 32-column chunk
-      const uint64_t sc2 = pack2(sc, sc), nm2 = pack2(neg_m, neg_m);
+      const uint64_t sc2 = pack2(scale2, scale2), nm2 = pack2(neg_m, neg_m);
       uint64_t sum2[4] = {0ull, 0ull, 0ull, 0ull};
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
