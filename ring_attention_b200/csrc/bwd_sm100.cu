@@ -454,29 +454,24 @@ __global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_con
     const int kv_row = kt * kTileRows + r;
     const float scale2 = p.scale * kLog2e;
     const bool alibi = (kinds & RA_MOD_ALIBI) != 0;
-    int32_t kpos = 0, kseg = 0;
-    bool kpre = false;
     const bool row_valid = !RAGGED || kv_row < p.lk;
+    // Score-mod inputs of this key row: read again for every tile that needs them (few do) instead of
+    // being held in registers that the loop is short of.
     const int64_t mod_row = (int64_t)bb * p.lk + (row_valid ? kv_row : p.lk - 1);
-    if (p.mod.kv_pos) kpos = p.mod.kv_pos[mod_row];
-    if (p.mod.kv_seg) kseg = p.mod.kv_seg[mod_row];
-    if (p.mod.kv_pre) kpre = p.mod.kv_pre[mod_row] != 0;
+    auto key_pos = [&]() { return p.mod.kv_pos ? __ldg(p.mod.kv_pos + mod_row) : 0; };
     bool ok = true;  // warp-uniform: the tile scan below votes across the warp
     float pf[64];        // P^T of the tile whose dS^T is formed next (this thread's row, 64 columns)
     uint32_t sv[2][32];
-    const float alibi_over_scale = alibi ? p.mod.slopes[hh] / p.scale : 0.f;
-    const float slope2 = alibi ? p.mod.slopes[hh] * kLog2e : 0.f;
     Window& win = win0;
 
     // One loop body serves every tile so that each phase exists once in the instruction
     // stream: step k does dS^T(k-1), then P^T(k).
-    int i_prev = -1, e_cur = next_active(win, first_tile), i_cur = e_cur & kTileIdx;
+    bool any = false;  // whether this CTA had any tile
+    int e_cur = next_active(win, first_tile), i_cur = e_cur & kTileIdx;
     int32_t q0_cur = win.hit_pos0;  // first query position of the tile (used when its positions are contiguous)
     for (int k = 0; ok; ++k) {
       const bool have_prev = k > 0, have_cur = i_cur < P.n_q_tiles;
       if (!have_prev && !have_cur) break;
-      const int e_next = have_cur ? next_active(win, i_cur + 1) : P.n_q_tiles;
-      const int32_t q0_next = win.hit_pos0;
       if (have_prev) {
         // ---- dS^T = P^T * (dP^T * scale - delta * scale) of tile k-1 -> shared memory, 128-byte swizzle
         const int n = k - 1, s = n & 1;
@@ -535,7 +530,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_con
         const int64_t q0 = (int64_t)bb * p.lq + (int64_t)i * kTileRows + g * 64;
         uint32_t vis[2];
         if (need_mask) {  // found while the scores are on their way
-          visible_columns<false>(vis, kinds, p.mod.window, kpos, kseg, kpre, p.mod.q_pos + q0, p.mod.q_seg + q0,
+          visible_columns<false>(vis, kinds, p.mod.window, key_pos(), p.mod.kv_seg ? __ldg(p.mod.kv_seg + mod_row) : 0,
+                                 p.mod.kv_pre && __ldg(p.mod.kv_pre + mod_row) != 0, p.mod.q_pos + q0, p.mod.q_seg + q0,
                                  p.mod.q_pre + q0, q0_cur + g * 64, (e_cur & kContigBit) != 0, RAGGED ? ncols : 64);
           if (RAGGED && !row_valid) vis[0] = vis[1] = 0u;
         }
@@ -544,7 +540,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_con
         if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[S_FULL], n & 1, abort_flag, P.status, kStBwdCompute)))) break;
         tc_fence_after();
         if (dense || (alibi && !alibi_inline)) {
-          bias_scores_tmem<false>(tmem_S + lane_off + g * 64, 64, alibi && !alibi_inline, alibi_over_scale, kpos,
+          bias_scores_tmem<false>(tmem_S + lane_off + g * 64, 64, alibi && !alibi_inline, alibi ? p.mod.slopes[hh] / p.scale : 0.f, key_pos(),
                                   p.mod.q_pos + q0,
                                   dense ? p.mod.bias + (int64_t)bb * p.mod.bsb + (int64_t)hh * p.mod.bsh +
                                               ((int64_t)i * kTileRows + g * 64) * p.mod.bsq + kv_row
@@ -558,7 +554,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_con
         if (alibi_inline) {
           // scale * s - slope * (q_pos - kv_pos), times log2(e), with q_pos = q0 + column; the
           // position differences are exact in fp32
-          const float rr = slope2 * (float)(kpos - (q0_cur + g * 64));
+          const float slope2 = p.mod.slopes[hh] * kLog2e;
+          const float rr = slope2 * (float)(key_pos() - (q0_cur + g * 64));
 #pragma unroll
           for (int c = 0; c < 64; ++c)
             sv[c >> 5][c & 31] = __float_as_uint(fmaf(-slope2, (float)c, fmaf(__uint_as_float(sv[c >> 5][c & 31]), scale2, rr)));
@@ -620,12 +617,12 @@ __global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_con
         mbar_arrive(&bars[P_READY]);
       }
       if (!have_cur) break;
-      i_prev = i_cur;
-      e_cur = e_next;
+      any = true;
+      e_cur = next_active(win, i_cur + 1);
       i_cur = e_cur & kTileIdx;
-      q0_cur = q0_next;
+      q0_cur = win.hit_pos0;
     }
-    const int n = (i_prev >= 0) ? 1 : 0;  // whether this CTA had any tile
+    const int n = any ? 1 : 0;
     // ---- epilogue: dK, dV of this K/V tile
     if (ok && n > 0) ok = mbar_wait(&bars[DKDV_FULL], 0, abort_flag, P.status, kStBwdCompute);
     if (ok && n > 0) {
