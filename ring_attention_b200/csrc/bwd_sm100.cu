@@ -459,7 +459,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_con
     // being held in registers that the loop is short of.
     const int64_t mod_row = (int64_t)bb * p.lk + (row_valid ? kv_row : p.lk - 1);
     auto key_pos = [&]() { return p.mod.kv_pos ? __ldg(p.mod.kv_pos + mod_row) : 0; };
-    bool ok = true;  // warp-uniform: the tile scan below votes across the warp
+    bool ok = true;  // warp-uniform: the tile scan below votes across the warp, TMEM loads take all of it
     float pf[64];        // P^T of the tile whose dS^T is formed next (this thread's row, 64 columns)
     uint32_t sv[2][32];
     Window& win = win0;
@@ -624,7 +624,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_con
     }
     const int n = any ? 1 : 0;
     // ---- epilogue: dK, dV of this K/V tile
-    if (ok && n > 0) ok = mbar_wait(&bars[DKDV_FULL], 0, abort_flag, P.status, kStBwdCompute);
+    if (ok && n > 0) ok = __all_sync(0xffffffffu, mbar_wait(&bars[DKDV_FULL], 0, abort_flag, P.status, kStBwdCompute));
     if (ok && n > 0) {
       tc_fence_after();
       constexpr int HALF = D / 2;

@@ -76,6 +76,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
   constexpr int PANELS = D / 64;           // 64-element (128-byte) panels per row
   constexpr int PANEL_BYTES = kTileRows * 128;
   constexpr int kPolyPairs = RAGGED ? 0 : poly_pairs(D);
+  // Which form of the wait for S (below): a vote costs head dim 128 nothing (32k causal tokens 8345 us, 8418 without
+  // it), head dim 64 and the ragged forms 1 to 6 % (8k causal, d 64: 438 against 425 us; 3001 causal, d 128: 152, 145).
+  constexpr bool kVoteOnS = D == 128 && !RAGGED;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;
@@ -287,7 +290,6 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
     if (p.mod.q_seg) qseg = p.mod.q_seg[mod_row];
     if (p.mod.q_pre) qpre = p.mod.q_pre[mod_row] != 0;
     const bool alibi = (kinds & RA_MOD_ALIBI) != 0;
-    bool ok = true;
 
     const float alibi_over_scale = alibi ? p.mod.slopes[hh] / p.scale : 0.f;
     const float slope2 = alibi ? p.mod.slopes[hh] * kLog2e : 0.f;
@@ -312,7 +314,15 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
       if (need_mask)  // a tile that mixes visible and masked pairs: found while its scores are on their way
         visible_columns<true>(vis, kinds, p.mod.window, qpos, qseg, qpre, p.mod.kv_pos + kv0, p.mod.kv_seg + kv0,
                               p.mod.kv_pre + kv0, k0, kv_contig, ncols);
-      if (!(ok = mbar_wait(&bars[S_FULL0 + t], done & 1, abort_flag, P.status, kStFwdSoftmax))) break;
+      // A wait that runs out may do so for some lanes of a warp only, and what follows takes all 32 (TMEM
+      // loads, votes): no lane leaves on its own result.  Either the lanes vote, or nobody leaves: a lane that gives up
+      // finds or sets the abort flag, so the tiles that are left pass without a long wait and the epilogue, which
+      // looks at the flag, stores nothing.
+      if constexpr (kVoteOnS) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&bars[S_FULL0 + t], done & 1, abort_flag, P.status, kStFwdSoftmax))) break;
+      } else {
+        mbar_wait(&bars[S_FULL0 + t], done & 1, abort_flag, P.status, kStFwdSoftmax);
+      }
       tc_fence_after();
       if (dense || (alibi && !alibi_inline)) {
         bias_scores_tmem<true>(tmem_S[t] + lane_off, kTileRows, alibi && !alibi_inline, alibi_over_scale, qpos,
@@ -415,7 +425,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
 
     // Epilogue: fold in the carried state of earlier ring steps, bring (o, m, l) to the
     // exact running max, store.
-    if (ok && count > 0) ok = mbar_wait(&bars[O_FULL], 0, abort_flag, P.status, kStFwdSoftmax);
+    const bool ok = count == 0 || __all_sync(0xffffffffu, mbar_wait(&bars[O_FULL], 0, abort_flag, P.status, kStFwdSoftmax) && *abort_flag == 0);
     if (ok) {
       tc_fence_after();
       const float beta = (m_ref == -INFINITY) ? 1.f : ex2(m_ref - m_true);
