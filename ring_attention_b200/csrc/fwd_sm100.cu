@@ -45,10 +45,13 @@ constexpr int kFwdThreads = 384, kRegsSoftmax = 216, kRegsOther = 72;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kRescaleThreshold = 8.0f;  // log2 units: P stays below 2^8
 // Of every 16 column pairs of the softmax, how many get their exponentials from the polynomial
-// on the FMA pipe (the others use ex2 on the special-function unit).  Forward of 32k causal tokens,
-// d 128, with 0 / 2 / 3 / 4 / 5 / 6 pairs: 7.85 / 7.99 / 7.55 / 7.44 / 8.55 / 8.07 ms; of 64k windowed
-// tokens, d 64: 7.63 / 7.70 / 7.78 / 7.81 / 8.02 / 8.61 ms (tiles with half the MMA time gain nothing).
-__host__ __device__ constexpr int poly_pairs(int d) { return d == 128 ? 4 : 0; }
+// on the FMA pipe (the others use ex2 on the special-function unit).  Measured per value, two to three
+// alternating runs each, which agree to 0.5 % (us; SM clock 1965 MHz unless noted):
+//   d 128, 32k causal tokens, b 2, h 16 (power cap, 1500 to 1580 MHz): 3: 8435, 4: 8370, 5: 9025, 6: 9055;
+//   d 128, 4k causal, b 4, h 16 (power cap, 1650 to 1700 MHz): 3: 344, 4: 341, 5: 365, 6: 367;
+//   d 64, 8k causal, b 2, h 16: 0: 459, 2: 425, 3: 428; 64k windowed ALiBi, b 4, h 16: 0: 7080, 2: 7035, 3: 7090;
+//   d 64 without masks (PLAIN), 6144 tokens, b 1, h 16: 0: 238, 2: 246, 3: 237, 4: 236; 4k, b 4: 394, 405, 400, 400.
+__host__ __device__ constexpr int poly_pairs(int d, bool plain) { return d == 128 ? 4 : (plain ? 0 : 2); }
 
 struct FwdTcParams {
   CUtensorMap map_q, map_k, map_v;
@@ -70,12 +73,15 @@ enum Bar {
   S_FULL0, S_FULL1, P_FULL0, P_FULL1, O_FULL, NUM_BARS
 };
 
-template <int D, bool RAGGED>
+// PLAIN: a call without score-mods.  Its loop holds no mask code; at head dim 64, where the softmax warps are what
+// the kernel waits for, carrying that code cost 8 % (6144 tokens, b 1, h 16: 260 -> 238 us; at head dim 128 the
+// masked form serves such calls, 309 against 302 us).
+template <int D, bool RAGGED, bool PLAIN = false>
 __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_constant__ FwdTcParams P) {
   constexpr int TILE_BYTES = kTileRows * D * 2;
   constexpr int PANELS = D / 64;           // 64-element (128-byte) panels per row
   constexpr int PANEL_BYTES = kTileRows * 128;
-  constexpr int kPolyPairs = RAGGED ? 0 : poly_pairs(D);
+  constexpr int kPolyPairs = RAGGED ? 0 : poly_pairs(D, PLAIN);
   // Which form of the wait for S (below): a vote costs head dim 128 nothing (32k causal tokens 8345 us, 8418 without
   // it), head dim 64 and the ragged forms 1 to 6 % (8k causal, d 64: 438 against 425 us; 3001 causal, d 128: 152, 145).
   constexpr bool kVoteOnS = D == 128 && !RAGGED;
@@ -100,7 +106,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
   const int hh = bh % p.h, bb = bh / p.h;
   const int qt0 = pair * 2;
   const int ntile = (qt0 + 1 < P.n_q_tiles) ? 2 : 1;
-  const uint32_t kinds = p.mod.kinds;
+  const uint32_t kinds = PLAIN ? 0u : p.mod.kinds;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < NUM_BARS; ++i) {
@@ -294,20 +300,20 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
     const float alibi_over_scale = alibi ? p.mod.slopes[hh] / p.scale : 0.f;
     const float slope2 = alibi ? p.mod.slopes[hh] * kLog2e : 0.f;
     // first position of the K/V tile the loop is about to visit, read one tile ahead
-    const bool has_pos = p.mod.kv_pos != nullptr;
+    const bool has_pos = !PLAIN && p.mod.kv_pos != nullptr;
     int32_t k0_next = (has_pos && count > 0) ? p.mod.kv_pos[(int64_t)bb * p.lk + (int64_t)(list[0] & kTileIdx) * kTileRows] : 0;
     int done = 0;  // K/V tiles this query tile has been through
     for (int i = 0; i < count; ++i) {
       const uint32_t entry = list[i];
       const int j = entry & kTileIdx;
-      const bool need_mask = (entry & (kMixed << t)) != 0;
+      const bool need_mask = !PLAIN && (entry & (kMixed << t)) != 0;
       // ALiBi over a tile of contiguous key positions is two FMAs per score in registers, over
       // scattered ones it takes the in-TMEM pass below
       const bool kv_contig = (entry & kContig) != 0;
       const bool alibi_inline = alibi && kv_contig;
       const int32_t k0 = k0_next;
       if (has_pos && i + 1 < count) k0_next = p.mod.kv_pos[(int64_t)bb * p.lk + (int64_t)(list[i + 1] & kTileIdx) * kTileRows];
-      if (!(entry & (kVisible << t))) continue;
+      if (!PLAIN && !(entry & (kVisible << t))) continue;
       const int64_t kv0 = (int64_t)bb * p.lk + (int64_t)j * kTileRows;
       const int ncols = RAGGED ? min(kTileRows, p.lk - j * kTileRows) : kTileRows;  // key rows of this tile
       uint32_t vis[4];
@@ -579,17 +585,24 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-template <int D, bool RAGGED>
+template <int D, bool RAGGED, bool PLAIN = false>
 cudaError_t launch_fwd(const FwdTcParams& P, cudaStream_t s) {
   constexpr size_t kSmem = 6 * kTileRows * D * 2 + kMaxTiles * 5 + NUM_BARS * 8 + 64 + 1024;
   constexpr size_t kRequest = kSmem < 120 * 1024 ? 120 * 1024 : kSmem;  // one CTA per SM: it owns all of TMEM
-  auto kern = tc_fwd_kernel<D, RAGGED>;
+  auto kern = tc_fwd_kernel<D, RAGGED, PLAIN>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRequest);
   if (e != cudaSuccess) return e;
   const int n_pairs = (P.n_q_tiles + 1) / 2;
   kern<<<n_pairs * P.p.b * P.p.h, kFwdThreads, kRequest, s>>>(P);
   count_launch();
   return cudaGetLastError();
+}
+
+// Lengths that are multiples of 128.
+cudaError_t launch_fwd_aligned(const FwdTcParams& P, cudaStream_t s) {
+  if (P.p.dk == 128) return launch_fwd<128, false>(P, s);
+  const bool plain = (P.p.mod.kinds & (kMetaKinds | RA_MOD_DENSE)) == 0;
+  return plain ? launch_fwd<64, false, true>(P, s) : launch_fwd<64, false>(P, s);
 }
 
 }  // namespace
@@ -727,7 +740,7 @@ cudaError_t tc_fwd_block(const FwdParams& p, cudaStream_t s) {
   const bool ragged = p.lq % kTileRows || p.lk % kTileRows;
   if (e == cudaSuccess) {
     if (ragged) e = p.dk == 128 ? launch_fwd<128, true>(P, s) : launch_fwd<64, true>(P, s);
-    else e = p.dk == 128 ? launch_fwd<128, false>(P, s) : launch_fwd<64, false>(P, s);
+    else e = launch_fwd_aligned(P, s);
   }
   if (meta) cudaFreeAsync(meta, s);  // stream-ordered: after the kernels above, also when one failed to launch
   return e;
@@ -842,7 +855,7 @@ extern "C" int ra_fwd_block_static(const ra_shape_t* shape, const ra_tensor_t* q
     P.meta_q = mq;
     P.meta_kv = mk;
   }
-  e = p.dk == 128 ? launch_fwd<128, false>(P, s) : launch_fwd<64, false>(P, s);
+  e = launch_fwd_aligned(P, s);
   if (e != cudaSuccess) return fail_cuda(e, "tcgen05 forward block (static scratch)");
   set_last_impl(RA_IMPL_TCGEN05);
   return 0;
