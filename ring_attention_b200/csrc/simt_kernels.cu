@@ -667,8 +667,12 @@ cudaError_t launch_bwd(const BwdParams& p, cudaStream_t s) {
 
 template <typename T>
 cudaError_t dispatch_fwd(const FwdParams& p, cudaStream_t s) {
+  // By dv alone: the accumulators and the staged V have that many columns, dk is walked in chunks.  dv 17
+  // to 128 comes here with dk above 128.
   int d = p.dv;
   if (d <= 16) return launch_fwd<T, 16>(p, s);
+  if (d <= 64) return launch_fwd<T, 64>(p, s);
+  if (d <= 128) return launch_fwd<T, 128>(p, s);
   return launch_fwd<T, 256>(p, s);
 }
 template <typename T>
