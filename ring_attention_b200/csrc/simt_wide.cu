@@ -35,37 +35,80 @@ __device__ __forceinline__ void cp_wait() {
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 
-// Rows [row0, row0 + rows) x D_PAD columns of an operand into shared memory as floats, zeros outside
-// the tensor.  fp32 rows on 16-byte boundaries go as asynchronous copies (the caller commits and
-// waits), anything else through registers.
-template <typename T, int D_PAD, int NT>
-__device__ __forceinline__ void stage_rows(float* dst, const T* base, int64_t sl, int row0, int nrows, int rows, int dim) {
-  constexpr int P = D_PAD + 4;
-  if constexpr (sizeof(T) == 4) {
-    if (((reinterpret_cast<uintptr_t>(base) | (uintptr_t)(sl * 4) | (uintptr_t)(dim * 4)) & 15) == 0) {
-      for (int e = threadIdx.x; e < rows * (D_PAD / 4); e += NT) {
-        const int r = e / (D_PAD / 4), c = (e % (D_PAD / 4)) * 4;
-        const bool in = row0 + r < nrows && c < dim;
-        const T* src = in ? base + (int64_t)(row0 + r) * sl + c : base;
-        const uint32_t n = in ? 16u : 0u;  // bytes read; the rest of the 16 is zero-filled
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ptx::smem_u32(dst + r * P + c)), "l"(src), "r"(n)
-                     : "memory");
+// Rows [row0, row0 + ROWS) x D_PAD columns of an operand into shared memory as floats, zeros outside
+// the tensor, in two halves so that the loads run under what stands between them: `begin` starts them,
+// `end` (after it, the tile's old contents no longer read) leaves the tile complete.  fp32 rows on 16-byte
+// boundaries go as asynchronous copies (the caller commits and waits); bf16 rows on 16-byte boundaries
+// wait in registers, 16 bytes a load (one element a load, complete in `begin`, made the forward at head
+// dims above 64 slower than the general kernel: 1000 x 1000, 8 heads, d 96: 370 against 268 us);
+// anything else element by element, all in `begin`.
+template <typename T, int D_PAD, int NT, int ROWS>
+struct Stage {
+  static constexpr int P = D_PAD + 4;
+  static constexpr int N16 = sizeof(T) == 2 ? ROWS * (D_PAD / 8) / NT : 1;  // 16-byte loads of a thread
+  static_assert(sizeof(T) == 4 || ROWS * (D_PAD / 8) % NT == 0, "uneven share");
+  uint4 held[N16];
+  bool holding = false;
+
+  __device__ __forceinline__ void begin(float* dst, const T* base, int64_t sl, int row0, int nrows, int dim) {
+    const bool aligned =
+        ((reinterpret_cast<uintptr_t>(base) | (uintptr_t)(sl * sizeof(T)) | (uintptr_t)(dim * sizeof(T))) & 15) == 0;
+    if (aligned) {
+      if constexpr (sizeof(T) == 4) {
+        for (int e = threadIdx.x; e < ROWS * (D_PAD / 4); e += NT) {
+          const int r = e / (D_PAD / 4), c = (e % (D_PAD / 4)) * 4;
+          const bool in = row0 + r < nrows && c < dim;
+          const T* src = in ? base + (int64_t)(row0 + r) * sl + c : base;
+          const uint32_t n = in ? 16u : 0u;  // bytes read; the rest of the 16 is zero-filled
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ptx::smem_u32(dst + r * P + c)), "l"(src), "r"(n)
+                       : "memory");
+        }
+      } else {
+        holding = true;
+#pragma unroll
+        for (int i = 0; i < N16; ++i) {
+          const int e = threadIdx.x + i * NT, r = e / (D_PAD / 8), c = (e % (D_PAD / 8)) * 8;
+          held[i] = (row0 + r < nrows && c < dim) ? *reinterpret_cast<const uint4*>(base + (int64_t)(row0 + r) * sl + c)
+                                                  : make_uint4(0u, 0u, 0u, 0u);
+        }
       }
       return;
     }
+    for (int e = threadIdx.x; e < ROWS * D_PAD; e += NT) {
+      const int r = e / D_PAD, c = e % D_PAD;
+      dst[r * P + c] = (row0 + r < nrows && c < dim) ? load_as_float(base + (int64_t)(row0 + r) * sl + c) : 0.f;
+    }
   }
-  for (int e = threadIdx.x; e < rows * D_PAD; e += NT) {
-    const int r = e / D_PAD, c = e % D_PAD;
-    dst[r * P + c] = (row0 + r < nrows && c < dim) ? load_as_float(base + (int64_t)(row0 + r) * sl + c) : 0.f;
+  __device__ __forceinline__ void end(float* dst) {
+    if constexpr (sizeof(T) == 2) {
+      if (!holding) return;
+      holding = false;
+#pragma unroll
+      for (int i = 0; i < N16; ++i) {
+        const int e = threadIdx.x + i * NT, r = e / (D_PAD / 8), c = (e % (D_PAD / 8)) * 8;
+        const uint4 v = held[i];
+        float4* to = reinterpret_cast<float4*>(dst + r * P + c);
+        to[0] = make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16),
+                            __uint_as_float(v.y & 0xffff0000u));
+        to[1] = make_float4(__uint_as_float(v.z << 16), __uint_as_float(v.z & 0xffff0000u), __uint_as_float(v.w << 16),
+                            __uint_as_float(v.w & 0xffff0000u));
+      }
+    }
   }
-}
+  __device__ __forceinline__ void whole(float* dst, const T* base, int64_t sl, int row0, int nrows, int dim) {
+    begin(dst, base, sl, row0, nrows, dim);
+    end(dst);
+  }
+};
 
-// acc[i][j] += (even, odd) halves of sum_c A[R ty + i][c] * B[tx + 16 j][c]
+// acc[i][j] += (even, odd) halves of sum_c A[R ty + i][c] * B[tx + 16 j][c] over the first `dim` columns
+// (rounded up to 16: the rest are zeros)
 template <int D_PAD, int R>
-__device__ __forceinline__ void dot_tile(uint64_t (&acc)[R][4], const float* A, const float* B, int ty, int tx) {
+__device__ __forceinline__ void dot_tile(uint64_t (&acc)[R][4], const float* A, const float* B, int dim, int ty, int tx) {
   constexpr int P = D_PAD + 4;
+  const int cols = (dim + 15) & ~15;
 #pragma unroll 4
-  for (int c = 0; c < D_PAD; c += 4) {
+  for (int c = 0; c < cols; c += 4) {
     ulonglong2 a[R], b[4];
 #pragma unroll
     for (int i = 0; i < R; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(A + (ty * R + i) * P + c);
@@ -306,7 +349,8 @@ __global__ void __launch_bounds__(16 * TY, D_PAD == 64 ? 2 : 1) wide_fwd_kernel(
       o_acc[i][n] = pack2(v[0], v[1]);
     }
   }
-  stage_rows<T, D_PAD, NT>(Qs, qb, p.q.sl, q0, p.lq, BM, p.dk);
+  Stage<T, D_PAD, NT, BM>().whole(Qs, qb, p.q.sl, q0, p.lq, p.dk);
+  Stage<T, D_PAD, NT, BT> stage_k, stage_v;
 
   const int n_tiles = (p.lk + BT - 1) / BT;
   for (int base = 0; base < n_tiles; base += kClsTiles) {
@@ -319,11 +363,11 @@ __global__ void __launch_bounds__(16 * TY, D_PAD == 64 ? 2 : 1) wide_fwd_kernel(
       return t;
     };
     int t = next(0);
-    if (t < end) stage_rows<T, D_PAD, NT>(Ks, kb, p.k.sl, (base + t) * BT, p.lk, BT, p.dk);
+    if (t < end) stage_k.whole(Ks, kb, p.k.sl, (base + t) * BT, p.lk, p.dk);
     cp_commit();
     while (t < end) {
       const int k0 = (base + t) * BT, tn = next(t + 1);
-      stage_rows<T, D_PAD, NT>(Vs, vb, p.v.sl, k0, p.lk, BT, p.dv);
+      stage_v.begin(Vs, vb, p.v.sl, k0, p.lk, p.dv);
       cp_commit();
       cp_wait<1>();
       __syncthreads();
@@ -332,9 +376,10 @@ __global__ void __launch_bounds__(16 * TY, D_PAD == 64 ? 2 : 1) wide_fwd_kernel(
       for (int i = 0; i < R; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
-      dot_tile<D_PAD, R>(acc, Qs, Ks, ty, tx);
+      dot_tile<D_PAD, R>(acc, Qs, Ks, p.dk, ty, tx);
+      stage_v.end(Vs);
       __syncthreads();
-      if (tn < end) stage_rows<T, D_PAD, NT>(Ks, kb, p.k.sl, (base + tn) * BT, p.lk, BT, p.dk);
+      if (tn < end) stage_k.begin(Ks, kb, p.k.sl, (base + tn) * BT, p.lk, p.dk);
       cp_commit();
       float s[R][4];
       score_patch<R>(s, acc, p.mod, qm, km, p.scale, slope, cls[t] == 2 || (p.mod.kinds & RA_MOD_ALIBI), bb, hh, q0, k0, ty, tx);
@@ -358,6 +403,7 @@ __global__ void __launch_bounds__(16 * TY, D_PAD == 64 ? 2 : 1) wide_fwd_kernel(
 #pragma unroll
         for (int n = 0; n < NO; ++n) o_acc[i][n] = ptx::mul2(o_acc[i][n], c2);  // ring.py:72
       }
+      stage_k.end(Ks);
       cp_wait<1>();
       __syncthreads();
       mul_rows<D_PAD, R>(o_acc, Ps, Vs, ty, tx);
@@ -462,8 +508,8 @@ __global__ void __launch_bounds__(16 * TY, D_PAD == 64 ? 2 : 1) wide_bwd_kernel(
   for (int i = 0; i < R; ++i)
 #pragma unroll
     for (int n = 0; n < NO; ++n) dk_acc[i][n] = dv_acc[i][n] = 0ull;
-  stage_rows<T, D_PAD, NT>(Ks, kb, p.k.sl, k0, p.lk, BT, p.dk_dim);
-  stage_rows<T, D_PAD, NT>(Vs, vb, p.v.sl, k0, p.lk, BT, p.dv_dim);
+  Stage<T, D_PAD, NT, BT>().whole(Ks, kb, p.k.sl, k0, p.lk, p.dk_dim);
+  Stage<T, D_PAD, NT, BT>().whole(Vs, vb, p.v.sl, k0, p.lk, p.dv_dim);
 
   const int n_tiles = (p.lq + BT - 1) / BT;
   for (int base = 0; base < n_tiles; base += kClsTiles) {
@@ -478,8 +524,8 @@ __global__ void __launch_bounds__(16 * TY, D_PAD == 64 ? 2 : 1) wide_bwd_kernel(
     float L_next = 0.f, delta_next = 0.f;
     auto stage_q = [&](int t) {
       const int q0 = (base + t) * BT;
-      stage_rows<T, D_PAD, NT>(Qs, qb, p.q.sl, q0, p.lq, BT, p.dk_dim);
-      stage_rows<T, D_PAD, NT>(Gs, gb, p.dout.sl, q0, p.lq, BT, p.dv_dim);
+      Stage<T, D_PAD, NT, BT>().whole(Qs, qb, p.q.sl, q0, p.lq, p.dk_dim);
+      Stage<T, D_PAD, NT, BT>().whole(Gs, gb, p.dout.sl, q0, p.lq, p.dv_dim);
       if (tid < BT && q0 + tid < p.lq) {
         L_next = p.lse[qrow_base + q0 + tid];
         delta_next = p.delta[qrow_base + q0 + tid];
@@ -501,8 +547,8 @@ __global__ void __launch_bounds__(16 * TY, D_PAD == 64 ? 2 : 1) wide_bwd_kernel(
       for (int i = 0; i < R; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = dacc[i][j] = 0ull;
-      dot_tile<D_PAD, R>(acc, Qs, Ks, ty, tx);   // S = Q K^T
-      dot_tile<D_PAD, R>(dacc, Gs, Vs, ty, tx);  // dP = dO V^T
+      dot_tile<D_PAD, R>(acc, Qs, Ks, p.dk_dim, ty, tx);   // S = Q K^T
+      dot_tile<D_PAD, R>(dacc, Gs, Vs, p.dv_dim, ty, tx);  // dP = dO V^T
       float s[R][4];
       score_patch<R>(s, acc, p.mod, qm, km, p.scale, slope, cls[t] == 2 || (p.mod.kinds & RA_MOD_ALIBI), bb, hh, q0, k0, ty, tx);
 #pragma unroll

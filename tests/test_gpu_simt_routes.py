@@ -44,6 +44,17 @@ def test_a_forward_pays_for_its_own_value_columns(dk, dv):
     assert _forward_ms(2, 4, 1500, dk, dv) < 0.8 * _forward_ms(2, 4, 1500, dk, 256)
 
 
+def test_a_forward_pays_for_its_own_key_columns():
+    # Q K^T over 128 padded columns instead of 16: equal times
+    assert _forward_ms(2, 4, 1500, 8, 128) < 0.85 * _forward_ms(2, 4, 1500, 128, 128)
+
+
+@pytest.mark.parametrize("d", [80, 128])
+def test_a_forward_on_bf16_inputs_costs_no_more_than_on_float32(d):
+    # staged element by element, bf16 tiles took 1.5 times the time of float32 ones
+    assert _forward_ms(1, 8, 1000, d, d, torch.bfloat16) < 1.25 * _forward_ms(1, 8, 1000, d, d)
+
+
 @pytest.mark.parametrize("dk,dv", [(160, 32), (256, 64), (192, 128), (8, 128), (20, 100)])
 def test_those_head_dims_against_the_oracle(dk, dv):
     q, k, v, do, _ = make_inputs(dk, 2, 130, 200, 2, dk, torch.float32, dv=dv)
