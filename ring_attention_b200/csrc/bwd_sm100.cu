@@ -53,6 +53,14 @@ constexpr int kBwdThreads = 512;  // four warpgroups: two of compute, the drain,
 // warp and one of the others, 2 * 152 + 152 + 56 = 512 = 16384 / 32.
 constexpr int kRegsCompute = 152, kRegsDrain = 152, kRegsOther = 56;
 
+// Ragged forms: the tensor pipe truncates every sum it accumulates, about 2^-24 of the sum each time and
+// always towards zero, 16 times per query tile with two-part P and dS.  The CUDA cores, which these calls used to
+// run on, round to nearest, so dK and dV move to fp32 sums in global memory after this many query tiles: p.dk and
+// p.dv, where a key tile's n rows are held as [D / 4][n] 16-byte chunks, so that a warp's accesses are contiguous.
+// 20001 causal tokens, d 128: relative error of dK 1.6640e-3 without that, 1.6625e-3 with it and on the CUDA cores;
+// 3001 causal, b 2, h 16: 467 -> 486 us.
+constexpr int kFlushTiles = 16;
+
 __host__ __device__ constexpr int bwd_do_stages(int d, bool ragged) { return ragged && d == 128 ? 1 : 2; }
 
 constexpr float kLog2e = 1.4426950408889634f;
@@ -70,7 +78,7 @@ struct BwdTcParams {
 
 enum Bar {
   KV_FULL = 0, Q_FULL0, Q_FULL1, Q_EMPTY0, Q_EMPTY1, DO_FULL0, DO_FULL1, DO_EMPTY0, DO_EMPTY1, S_FULL, DP_FULL, P_READY, DS_READY,
-  DQ_FULL, DQ_DRAINED, DKDV_FULL, NUM_BARS
+  DQ_FULL, DQ_DRAINED, DKDV_FULL, ACC_FULL, ACC_FLUSHED, NUM_BARS
 };
 
 __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
@@ -125,7 +133,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_con
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < NUM_BARS; ++i) {
-      uint32_t cnt = (i == P_READY || i == DS_READY) ? 256u : (i == DQ_DRAINED) ? 128u : 1u;
+      uint32_t cnt = (i == P_READY || i == DS_READY) ? 256u : (i == DQ_DRAINED || i == ACC_FLUSHED) ? 128u : 1u;
       mbar_init(&bars[i], cnt);
     }
     *abort_flag = (smem_u32(smem) & 1023u) ? 1u : 0u;  // the swizzled tiles need a 1024-byte aligned base
@@ -389,7 +397,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_con
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk)
               mma_ss_warp(tmem_dK, desc_from_lo(a0 + km_off(kk)), desc_from_lo(b0 + mn_off(kk)), idesc_dv,
-                     (n > 0) || kk > 0);
+                     (RAGGED ? n % kFlushTiles != 0 : n > 0) || kk > 0);
             if constexpr (RAGGED) {
 #pragma unroll
               for (int kk = 0; kk < 8; ++kk)
@@ -398,6 +406,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_con
           }
           tc_commit_warp(&bars[Q_EMPTY0 + s]);
           if (!has_next) break;
+          const bool flush = RAGGED && (n + 1) % kFlushTiles == 0;  // dV and dK start afresh with tile n + 1
+          if (flush) tc_commit_warp(&bars[ACC_FULL]);
           if constexpr (!SEP_DQ) {
             if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[DQ_DRAINED], par, abort_flag, P.status, kStBwdMma)))) break;
             if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[DO_FULL0 + dsn], dphn, abort_flag, P.status, kStBwdMma)))) break;
@@ -405,8 +415,9 @@ __global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_con
             issue_dp(dsn);
           }
           if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[P_READY], par ^ 1, abort_flag, P.status, kStBwdMma)))) break;
+          if (flush && !(ok = __all_sync(0xffffffffu, mbar_wait(&bars[ACC_FLUSHED], ((n + 1) / kFlushTiles - 1) & 1, abort_flag, P.status, kStBwdMma)))) break;
           tc_fence_after();
-          issue_dv(dsn, false);
+          issue_dv(dsn, flush);
           tc_commit_warp(&bars[DO_EMPTY0 + dsn]);
           i = inext;
         }
@@ -444,6 +455,36 @@ __global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_con
         if (!RAGGED || c < q_left)
           asm volatile("red.global.add.f32 [%0], %1;" ::"l"(base + c * D), "f"(__uint_as_float(dv[c >> 5][c & 31])) : "memory");
       i = next_active(win, i + 1) & kTileIdx;
+      if constexpr (RAGGED) {
+        if ((n + 1) % kFlushTiles == 0 && i < P.n_q_tiles) {
+          // dV, dK of the last kFlushTiles tiles to this thread's key row of the fp32 sums (nobody else adds to it)
+          if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[ACC_FULL], ((n + 1) / kFlushTiles - 1) & 1, abort_flag, P.status, kStBwdCompute)))) break;
+          tc_fence_after();
+          const int row = (warp & 3) * 32 + lane, rows = min(kTileRows, p.lk - kt * kTileRows);
+          const int64_t tile = (((int64_t)bb * p.h + hh) * p.lk + kt * kTileRows) * D + row * 4;
+          const bool first_flush = n + 1 == kFlushTiles;
+#pragma unroll 1
+          for (int c = 0; c < 2 * D; c += 32) {
+            tmem_ld32(tmem_dV + lane_off + c, dv[0]);  // dK's columns follow dV's
+            tc_wait_ld();
+            float* sum = (c < D ? p.dv + c * rows : p.dk + (c - D) * rows) + tile;
+            if (row < rows) {
+#pragma unroll
+              for (int e = 0; e < 32; e += 4) {
+                float* to = sum + e * rows;
+                if (first_flush)
+                  *reinterpret_cast<uint4*>(to) = make_uint4(dv[0][e], dv[0][e + 1], dv[0][e + 2], dv[0][e + 3]);
+                else
+                  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(to), "f"(__uint_as_float(dv[0][e])),
+                               "f"(__uint_as_float(dv[0][e + 1])), "f"(__uint_as_float(dv[0][e + 2])), "f"(__uint_as_float(dv[0][e + 3]))
+                               : "memory");
+              }
+            }
+          }
+          tc_fence_before();
+          mbar_arrive(&bars[ACC_FLUSHED]);
+        }
+      }
     }
   } else {
     // ------------------------------------------------------------ compute (warps 0-7)
@@ -466,10 +507,10 @@ __global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_con
 
     // One loop body serves every tile so that each phase exists once in the instruction
     // stream: step k does dS^T(k-1), then P^T(k).
-    bool any = false;  // whether this CTA had any tile
+    int k = 0;  // after the loop: how many tiles this CTA had
     int e_cur = next_active(win, first_tile), i_cur = e_cur & kTileIdx;
     int32_t q0_cur = win.hit_pos0;  // first query position of the tile (used when its positions are contiguous)
-    for (int k = 0; ok; ++k) {
+    for (; ok; ++k) {
       const bool have_prev = k > 0, have_cur = i_cur < P.n_q_tiles;
       if (!have_prev && !have_cur) break;
       if (have_prev) {
@@ -617,21 +658,55 @@ __global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_con
         mbar_arrive(&bars[P_READY]);
       }
       if (!have_cur) break;
-      any = true;
       e_cur = next_active(win, i_cur + 1);
       i_cur = e_cur & kTileIdx;
       q0_cur = win.hit_pos0;
     }
-    const int n = any ? 1 : 0;
+    const int n = k > 0 ? 1 : 0;
     // ---- epilogue: dK, dV of this K/V tile
+    constexpr int kSumChunks = RAGGED ? D / 8 : 1;
+    float4 sum[kSumChunks];  // RAGGED: this row's half of the sum of earlier tiles
+    const int flushes = RAGGED && k > 0 ? (k - 1) / kFlushTiles : 0;
+    auto load_sum = [&](const float* sums) {
+      const int rows = min(kTileRows, p.lk - kt * kTileRows);
+      const float* from = sums + (((int64_t)bb * p.h + hh) * p.lk + kt * kTileRows) * D + r * 4 + g * (D / 2) * rows;
+#pragma unroll
+      for (int j = 0; j < kSumChunks; ++j)
+        sum[j] = flushes > 0 && row_valid ? __ldcg(reinterpret_cast<const float4*>(from + 4 * j * rows)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    if constexpr (RAGGED) {  // dK's is on its way while the last MMAs run
+      if (ok && flushes > 0) ok = __all_sync(0xffffffffu, mbar_wait(&bars[ACC_FLUSHED], (flushes - 1) & 1, abort_flag, P.status, kStBwdCompute));
+      if (ok) load_sum(p.dk);
+    }
     if (ok && n > 0) ok = __all_sync(0xffffffffu, mbar_wait(&bars[DKDV_FULL], 0, abort_flag, P.status, kStBwdCompute));
-    if (ok && n > 0) {
+    if (RAGGED && ok && n > 0) {
+      tc_fence_after();
+      auto put = [&](uint32_t tmem, const TensorView& out) {
+        __nv_bfloat16* to = (__nv_bfloat16*)out.ptr + (int64_t)bb * out.sb + (int64_t)kv_row * out.sl + (int64_t)hh * out.sh + g * (D / 2);
+#pragma unroll
+        for (int j = 0; j + 1 < kSumChunks; j += 2) {
+          uint32_t a[8];
+          tmem_ld8(tmem + lane_off + g * (D / 2) + j * 4, a);
+          tc_wait_ld();
+          const float4 x = sum[j], y = sum[j + 1];
+          uint4 w;
+          w.x = pack_bf16(x.x + __uint_as_float(a[0]), x.y + __uint_as_float(a[1]));
+          w.y = pack_bf16(x.z + __uint_as_float(a[2]), x.w + __uint_as_float(a[3]));
+          w.z = pack_bf16(y.x + __uint_as_float(a[4]), y.y + __uint_as_float(a[5]));
+          w.w = pack_bf16(y.z + __uint_as_float(a[6]), y.w + __uint_as_float(a[7]));
+          if (row_valid) *reinterpret_cast<uint4*>(to + j * 4) = w;
+        }
+      };
+      put(tmem_dK, p.dk_out);
+      load_sum(p.dv);
+      put(tmem_dV, p.dv_out);
+    } else if (!RAGGED && ok && n > 0) {
       tc_fence_after();
       constexpr int HALF = D / 2;
       const int64_t krow = ((int64_t)bb * p.h + hh) * p.lk + kv_row;
       float* dk_row = p.dk + krow * D + g * HALF;
       float* dv_row = p.dv + krow * D + g * HALF;
-      const bool direct = RAGGED || p.dk_out.ptr != nullptr;  // ring of one: results go out in the input dtype
+      const bool direct = p.dk_out.ptr != nullptr;  // ring of one: results go out in the input dtype
       const bool fresh = p.overwrite != 0;          // the fp32 buffers hold nothing yet: store, do not add
       __nv_bfloat16* dk_o = direct ? (__nv_bfloat16*)p.dk_out.ptr + (int64_t)bb * p.dk_out.sb +
                                          (int64_t)kv_row * p.dk_out.sl + (int64_t)hh * p.dk_out.sh + g * HALF
@@ -650,7 +725,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_con
           w.y = pack_bf16(__uint_as_float(a[2]), __uint_as_float(a[3]));
           w.z = pack_bf16(__uint_as_float(a[4]), __uint_as_float(a[5]));
           w.w = pack_bf16(__uint_as_float(a[6]), __uint_as_float(a[7]));
-          if (row_valid) *reinterpret_cast<uint4*>(dk_o + c * 8) = w;
+          *reinterpret_cast<uint4*>(dk_o + c * 8) = w;
         } else {
 #pragma unroll
           for (int e = 0; e < 8; e += 4) {
@@ -670,7 +745,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_con
           w.y = pack_bf16(__uint_as_float(a[2]), __uint_as_float(a[3]));
           w.z = pack_bf16(__uint_as_float(a[4]), __uint_as_float(a[5]));
           w.w = pack_bf16(__uint_as_float(a[6]), __uint_as_float(a[7]));
-          if (row_valid) *reinterpret_cast<uint4*>(dv_o + c * 8) = w;
+          *reinterpret_cast<uint4*>(dv_o + c * 8) = w;
         } else {
 #pragma unroll
           for (int e = 0; e < 8; e += 4) {

@@ -64,7 +64,8 @@ struct BwdParams {
   float scale;
   // Optional, honoured by the tcgen05 kernel only: when dk_out.ptr is set this call is the
   // whole backward for these keys (ring of one) and the kernel stores dK, dV in the input
-  // dtype straight to the result tensors; dk / dv above are then not touched.
+  // dtype straight to the result tensors; dk / dv above are then left alone, or hold sums of the
+  // kernel's own (lengths that are not multiples of 128).
   TensorView dk_out, dv_out;
   // Optional: dk / dv above hold nothing yet and this call defines them (stores instead of
   // read-add-write, zeros for key rows that no query sees), so the caller need not clear them.

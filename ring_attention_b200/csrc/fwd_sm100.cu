@@ -19,9 +19,9 @@
 // stored.  These calls used to run on the CUDA cores with P in fp32, so here P keeps 16 bits: it goes
 // to TMEM as two bf16 halves (hi in the first, lo in the second half of S's columns) and PV runs twice;
 // every exponential is ex2.  What bounds it is the same softmax path plus 1.5 times the MMAs.  Causal
-// 3001 tokens, b 2, h 16, d 128, forward + backward: 15.6 -> 0.62 ms; 448 x 1500, b 8, h 16, d 64: 4.0 ->
-// 0.33 ms.  Relative error against 64 bits over such sizes (the results' bf16 rounding): out 1.58e-3 to
-// 1.66e-3, gradients 1.66e-3 to 1.86e-3, the same to four digits as on the CUDA cores.
+// 3001 tokens, b 2, h 16, d 128, forward + backward: 15.6 -> 0.64 ms; 448 x 1500, b 8, h 16, d 64: 4.0 ->
+// 0.35 ms.  Relative error against 64 bits from 333 to 20001 tokens (the results' bf16 rounding): out 1.57e-3 to
+// 1.66e-3, gradients 1.64e-3 to 1.67e-3, the same to four digits as on the CUDA cores.
 // TMEM columns: S0 [0,128) S1 [128,256) O0 [256,256+D) O1 [256+D,256+2D).
 #include <cstdio>
 #include <cstring>
@@ -44,6 +44,13 @@ using namespace ptx;
 constexpr int kFwdThreads = 384, kRegsSoftmax = 216, kRegsOther = 72;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kRescaleThreshold = 8.0f;  // log2 units: P stays below 2^8
+// Ragged forms: the tensor pipe truncates every sum it accumulates, about 2^-24 of the sum each time and
+// always towards zero, 16 times per K/V tile with two-part P.  The CUDA cores, which these calls used to run on,
+// round to nearest, so O moves to an fp32 sum in global memory after this many tiles: p.o, where a query
+// tile's n rows are held as [D / 4][n] 16-byte chunks, so that a warp's accesses are contiguous.  9842 tokens, no
+// mask, d 128: out comes 2.3e-5 of itself too small without that, 1.0e-5 with it (CUDA cores 0.4e-5; the bf16
+// rounding hides factors below about 1e-5); 5454 tokens, b 2, h 8: 367 -> 394 us.
+constexpr int kFlushTiles = 32;
 // Of every 16 column pairs of the softmax, how many get their exponentials from the polynomial
 // on the FMA pipe (the others use ex2 on the special-function unit).  Measured per value, two to three
 // alternating runs each, which agree to 0.5 % (us; SM clock 1965 MHz unless noted):
@@ -72,6 +79,36 @@ enum Bar {
   Q_FULL0 = 0, Q_FULL1, K_FULL0, K_FULL1, K_EMPTY0, K_EMPTY1, V_FULL0, V_FULL1, V_EMPTY0, V_EMPTY1,
   S_FULL0, S_FULL1, P_FULL0, P_FULL1, O_FULL, NUM_BARS
 };
+
+// RAGGED: a row's O moves from tensor memory to its fp32 sum (chunk j of the row at sums + j * pitch), which was
+// scaled by `alpha` since the last move.  The warp calls it together; kept out of line, because the loop that
+// calls it is short of registers.
+template <int D>
+__device__ __noinline__ void move_o(uint32_t tmem, float* sums, int pitch, bool row_valid, bool flushed, float alpha) {
+  const bool rescale = __any_sync(0xffffffffu, flushed && alpha != 1.f);
+#pragma unroll 1
+  for (int c = 0; c < D / 32; ++c) {
+    uint32_t o[32];
+    tmem_ld32(tmem + c * 32, o);
+    tc_wait_ld();
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      float* to = sums + (c * 8 + e) * pitch;
+      float4 v = make_float4(__uint_as_float(o[4 * e]), __uint_as_float(o[4 * e + 1]), __uint_as_float(o[4 * e + 2]),
+                             __uint_as_float(o[4 * e + 3]));
+      if (!row_valid) continue;
+      if (flushed && !rescale) {
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(to), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+      } else {
+        if (flushed) {
+          const float4 sum = __ldcg(reinterpret_cast<const float4*>(to));
+          v = make_float4(fmaf(sum.x, alpha, v.x), fmaf(sum.y, alpha, v.y), fmaf(sum.z, alpha, v.z), fmaf(sum.w, alpha, v.w));
+        }
+        *reinterpret_cast<float4*>(to) = v;
+      }
+    }
+  }
+}
 
 // PLAIN: a call without score-mods.  Its loop holds no mask code; at head dim 64, where the softmax warps are what
 // the kernel waits for, carrying that code cost 8 % (6144 tokens, b 1, h 16: 260 -> 238 us; at head dim 128 the
@@ -123,7 +160,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
   }
   // List of K/V tiles this CTA visits (index and class bits, see kTileIdx ...).  Tiles masked for
   // both query tiles are left out; a tile masked for one of them is visited for the other only.
-  // Every thread classifies its share of the tiles (one round of loads for up to 320 tiles), then
+  // Every thread classifies its share of the tiles (one round of loads for up to 384 tiles), then
   // warp 0 compacts the classes in order.
   const bool masked = (kinds & kMetaKinds) != 0;
   const bool dense = !RAGGED && (kinds & RA_MOD_DENSE) != 0;
@@ -260,7 +297,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
           if (cur & (kVisible << t)) {
             if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[P_FULL0 + t], done[t] & 1, abort_flag, P.status, kStFwdMma)))) break;
             tc_fence_after();
-            issue_pv(t, s, done[t] == 0);
+            issue_pv(t, s, RAGGED ? done[t] % kFlushTiles == 0 : done[t] == 0);
             ++done[t];
           }
           if (t == ntile - 1) tc_commit_warp(&bars[V_EMPTY0 + s]);
@@ -303,11 +340,15 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
     const bool has_pos = !PLAIN && p.mod.kv_pos != nullptr;
     int32_t k0_next = (has_pos && count > 0) ? p.mod.kv_pos[(int64_t)bb * p.lk + (int64_t)(list[0] & kTileIdx) * kTileRows] : 0;
     int done = 0;  // K/V tiles this query tile has been through
+    // RAGGED: once more than kFlushTiles tiles are done p.o holds the sum of earlier ones, to be multiplied by
+    // alpha_total; this row's chunk j is at o_sum() + j * o_pitch()
+    auto o_pitch = [&]() { return 4 * min(kTileRows, p.lq - (qt0 + t) * kTileRows); };
+    auto o_sum = [&]() { return p.o + (((int64_t)bb * p.h + hh) * p.lq + (qt0 + t) * kTileRows) * D + row_in_tile * 4; };
     for (int i = 0; i < count; ++i) {
       const uint32_t entry = list[i];
       const int j = entry & kTileIdx;
       const bool need_mask = !PLAIN && (entry & (kMixed << t)) != 0;
-      // ALiBi over a tile of contiguous key positions is two FMAs per score in registers, over
+      // ALiBi over a tile of contiguous key positions is one FMA per score in registers, over
       // scattered ones it takes the in-TMEM pass below
       const bool kv_contig = (entry & kContig) != 0;
       const bool alibi_inline = alibi && kv_contig;
@@ -330,6 +371,13 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
         mbar_wait(&bars[S_FULL0 + t], done & 1, abort_flag, P.status, kStFwdSoftmax);
       }
       tc_fence_after();
+      if constexpr (RAGGED) {
+        // P V of the tiles before is complete (S of this one was issued behind it) and the next one starts O afresh
+        if (done > 0 && done % kFlushTiles == 0) {
+          move_o<D>(tmem_O[t] + lane_off, o_sum(), o_pitch(), row_valid, done > kFlushTiles, alpha_total);
+          alpha_total = 1.f;
+        }
+      }
       if (dense || (alibi && !alibi_inline)) {
         bias_scores_tmem<true>(tmem_S[t] + lane_off, kTileRows, alibi && !alibi_inline, alibi_over_scale, qpos,
                                p.mod.kv_pos + kv0,
@@ -378,7 +426,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
         m_ref = m_new;
         l_run *= alpha;
         alpha_total *= alpha;
-        if (done > 0) {  // O of this tile holds the sum over the tiles before this one
+        if (RAGGED ? done % kFlushTiles != 0 : done > 0) {  // O of this tile holds the sum over the tiles before this one
 #pragma unroll 1
           for (int c = 0; c < D / 16; ++c) {
             uint32_t o[16];
@@ -431,11 +479,20 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
 
     // Epilogue: fold in the carried state of earlier ring steps, bring (o, m, l) to the
     // exact running max, store.
+    constexpr int kSumChunks = RAGGED ? D / 4 : 1;
+    float4 sum[kSumChunks];  // RAGGED: the sum of earlier tiles, on its way while the last MMAs run
+    if constexpr (RAGGED) {
+#pragma unroll
+      for (int j = 0; j < kSumChunks; ++j)
+        sum[j] = done > kFlushTiles && row_valid ? __ldcg(reinterpret_cast<const float4*>(o_sum() + j * o_pitch()))
+                                                 : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
     const bool ok = count == 0 || __all_sync(0xffffffffu, mbar_wait(&bars[O_FULL], 0, abort_flag, P.status, kStFwdSoftmax) && *abort_flag == 0);
     if (ok) {
       tc_fence_after();
       const float beta = (m_ref == -INFINITY) ? 1.f : ex2(m_ref - m_true);
-      const bool first = RAGGED || p.first;  // a ragged call is the whole attention: no carried state, results go out
+      // a ragged call is the whole attention: no carried state but its own sum of earlier tiles, results go out
+      const bool first = RAGGED ? done <= kFlushTiles : p.first != 0;
       const float in_scale = first ? 0.f : alpha_total * beta;
       float* o_row = p.o + state_row * D;
       const bool finalize = RAGGED || p.final_out.ptr != nullptr;
@@ -444,7 +501,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
       __nv_bfloat16* out_row = finalize ? (__nv_bfloat16*)p.final_out.ptr + (int64_t)bb * p.final_out.sb +
                                               (int64_t)q_row * p.final_out.sl + (int64_t)hh * p.final_out.sh
                                         : nullptr;
-#pragma unroll 1
+#pragma unroll (RAGGED ? D / 8 : 1)
       for (int c = 0; c < D / 8; ++c) {
         uint32_t o[8];
         if (done > 0) {
@@ -458,7 +515,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
 #pragma unroll
         for (int e = 0; e < 8; e += 4) {
           float4 prev = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (!first) prev = *reinterpret_cast<const float4*>(o_row + c * 8 + e);
+          if (RAGGED) prev = sum[RAGGED ? c * 2 + e / 4 : 0];
+          else if (!first) prev = *reinterpret_cast<const float4*>(o_row + c * 8 + e);
           val[e] = __uint_as_float(o[e]) * beta + prev.x * in_scale;
           val[e + 1] = __uint_as_float(o[e + 1]) * beta + prev.y * in_scale;
           val[e + 2] = __uint_as_float(o[e + 2]) * beta + prev.z * in_scale;

@@ -100,6 +100,37 @@ def test_masks(mask, order, d):
         _agree(a, b_, name)
 
 
+@pytest.mark.parametrize("d", [64, 128])
+def test_long_sums_are_not_truncated(d):
+    """The tensor pipe cuts every sum it accumulates towards zero, so a long sum in tensor memory comes out too
+    small by a common factor; the kernels therefore move O, dK and dV to float32 sums every 32 (16) tiles.
+    The factor is measured against 64 bits over every element of the results.  Bound: 16 sums a tile, each cut by
+    2^-24 on average, over the tiles of one move; sums of one sign pattern grow from zero, half of that; plus
+    four standard deviations of what rounding the results to bf16 leaves in the factor."""
+    n, h = 16061, 2
+    g = torch.Generator("cuda").manual_seed(d)
+    q, k, v, do = (torch.randn((1, n, h, d), generator=g, device="cuda").to(BF) for _ in range(4))
+    t = [x.requires_grad_(True) for x in (q, k, v)]
+    out = ra().ring_attention(*t, "sp")
+    _, dk, dv = torch.autograd.grad(out, t, do)
+    got = [x.detach()[0].double() for x in (out, dk, dv)]
+    sums = torch.zeros((3, 3), dtype=torch.float64, device="cuda")
+    for hh in range(h):
+        Q, K, V, G = (x.detach()[0, :, hh].double() for x in (q, k, v, do))
+        O64, dK, dV = torch.empty_like(Q), torch.zeros_like(K), torch.zeros_like(V)
+        for r in (slice(i, min(i + 2048, n)) for i in range(0, n, 2048)):
+            P = (Q[r] @ K.T / d**0.5).softmax(-1)
+            O64[r] = P @ V
+            delta = (got[0][r, hh] * G[r]).sum(-1)  # from the rounded out, as the backward has it
+            dK += (P * (G[r] @ V.T - delta[:, None])).T @ Q[r] / d**0.5
+            dV += P.T @ G[r]
+        for i, want in enumerate((O64, dK, dV)):
+            err = got[i][:, hh] - want
+            sums[i] += torch.stack([(err * want).sum(), (want * want).sum(), (err * want).pow(2).sum()])
+    for name, tiles, (a, b, c) in zip(("out", "dk", "dv"), (32, 16, 16), sums.tolist()):
+        assert abs(a / b) < tiles * 16 * 2.0**-25 + 4 * c**0.5 / b, f"{name}: factor 1 {a / b:+.2e}"
+
+
 def test_named_implementation_still_refuses():
     q = torch.zeros((1, 100, 1, 64), dtype=BF, device="cuda")
     with pytest.raises(RuntimeError):
