@@ -4,10 +4,12 @@ test_bwd_protocol_model.py, whose barrier and buffer models it uses).
 
 Roles: the TMA producer (Q tiles once, then K and V of every visited K/V tile through two
 stages each), the MMA issuer (S = Q K^T for both query tiles of the CTA, O += P V), one
-softmax warpgroup per query tile.  The tensor pipe executes in issue order, so a commit
-covers everything issued before it: the softmax of step i may rescale O because S(i) was
-issued behind P V of step i-1 -- there is no barrier of its own for that, and the model checks
-that no rescale lands under a running P V.
+softmax warpgroup per query tile.  A K/V tile that is masked for one of the two query tiles is
+visited for the other one only, so every query tile counts its own steps (`done`) and the phases of
+its S_FULL and P_FULL follow that count, while the stages of K and V follow the CTA's list.  The
+tensor pipe executes in issue order, so a commit covers everything issued before it: the softmax of a
+step may rescale O because its S was issued behind the P V of the query tile's step before -- there
+is no barrier of its own for that, and the model checks that no rescale lands under a running P V.
 """
 import random
 
@@ -17,8 +19,11 @@ from tests.test_bwd_protocol_model import Barrier, Buffer
 
 
 class FwdCta:
-    def __init__(self, steps, ntile, rng, mutate=None):
-        self.n, self.ntile, self.rng, self.mutate = steps, ntile, rng, mutate
+    """`visible[i][t]`: query tile t sees something of the i-th K/V tile of the list."""
+
+    def __init__(self, visible, ntile, rng, mutate=None):
+        self.n, self.ntile, self.rng, self.mutate = len(visible), ntile, rng, mutate
+        self.visible = visible
         names = ["K_FULL0", "K_FULL1", "K_EMPTY0", "K_EMPTY1", "V_FULL0", "V_FULL1", "V_EMPTY0", "V_EMPTY1", "O_FULL"]
         for t in range(ntile):
             names += [f"Q_FULL{t}", f"S_FULL{t}", f"P_FULL{t}"]
@@ -84,18 +89,20 @@ class FwdCta:
             self.pipe.append(("mma", [(f"Q{t}", ("Q", t)), (f"K{i & 1}", ("K", i))], [(f"S{t}", ("S", t, i))]))
             self.pipe.append(("commit", f"S_FULL{t}"))
 
-        def issue_pv(t, i):
+        def issue_pv(t, i, done):
             # accumulates into O: it reads the O that the softmax of this step left, and writes
-            self.pipe.append(("mma", [(f"S{t}", ("P", t, i)), (f"V{i & 1}", ("V", i)), (f"O{t}", ("O", t, i - 1))],
-                              [(f"O{t}", ("O", t, i))]))
+            self.pipe.append(("mma", [(f"S{t}", ("P", t, i)), (f"V{i & 1}", ("V", i)), (f"O{t}", ("O", t, done - 1))],
+                              [(f"O{t}", ("O", t, done))]))
 
         for t in range(ntile):
             yield from self.wait(f"Q_FULL{t}", 0)
         yield from self.wait("K_FULL0", 0)
         for t in range(ntile):
-            issue_s(t, 0)
+            if self.visible[0][t]:
+                issue_s(t, 0)
         self.pipe.append(("commit", "K_EMPTY0"))
         yield "ran"
+        done = [0] * ntile
         for i in range(n):
             s, sn, ph, phn = i & 1, (i + 1) & 1, (i >> 1) & 1, ((i + 1) >> 1) & 1
             has_next = i + 1 < n
@@ -103,13 +110,16 @@ class FwdCta:
                 yield from self.wait(f"K_FULL{sn}", phn)
             yield from self.wait(f"V_FULL{s}", ph)
             for t in range(ntile):
-                if self.mutate != "no_p_full_wait":
-                    yield from self.wait(f"P_FULL{t}", i & 1)
-                issue_pv(t, i)
+                if self.visible[i][t]:
+                    if self.mutate != "no_p_full_wait":
+                        yield from self.wait(f"P_FULL{t}", (i if self.mutate == "p_full_parity_of_list" else done[t]) & 1)
+                    issue_pv(t, i, done[t])
+                    done[t] += 1
                 if t == ntile - 1:
                     self.pipe.append(("commit", f"V_EMPTY{s}"))
                 if has_next:
-                    issue_s(t, i + 1)
+                    if self.visible[i + 1][t]:
+                        issue_s(t, i + 1)
                     if t == ntile - 1:
                         self.pipe.append(("commit", f"K_EMPTY{sn}"))
                 yield "ran"
@@ -117,8 +127,11 @@ class FwdCta:
         yield "ran"
 
     def softmax(self, t):
+        done = 0
         for i in range(self.n):
-            par = (i & 1) ^ (1 if self.mutate == "s_full_parity" else 0)
+            if not self.visible[i][t]:
+                continue
+            par = ((i if self.mutate == "s_full_parity_of_list" else done) & 1) ^ (1 if self.mutate == "s_full_parity" else 0)
             yield from self.wait(f"S_FULL{t}", par)
             self.buf[f"S{t}"].begin_read(("S", t, i))
             yield "ran"
@@ -126,18 +139,30 @@ class FwdCta:
             # rescale of O (in the kernel only when the row max grew enough; here always): the
             # tile must hold P V of every earlier step and no P V may be running on it
             o = self.buf[f"O{t}"]
-            assert o.tag == ("O", t, i - 1), f"O{t}: rescale at step {i} finds {o.tag}"
-            o.write(("O", t, i - 1))
+            assert o.tag == ("O", t, done - 1), f"O{t}: rescale at step {i} finds {o.tag}"
+            o.write(("O", t, done - 1))
             self.buf[f"S{t}"].write(("P", t, i))
             self.bar[f"P_FULL{t}"].arrive()
+            done += 1
             yield "ran"
         yield from self.wait("O_FULL", 0)
-        assert self.buf[f"O{t}"].tag == ("O", t, self.n - 1)
+        assert self.buf[f"O{t}"].tag == ("O", t, done - 1)
 
 
-def run(steps, ntile, seed, mutate=None, max_steps=200000):
+def random_visibility(steps, ntile, rng):
+    """Lists as the kernel makes them: every listed tile is visible to at least one query tile.  Runs of
+    tiles that only one of them sees (a window's two ends, a causal diagonal, documents) among others."""
+    choices = [(True,)] if ntile == 1 else [(True, True), (True, False), (False, True)]
+    out = []
+    while len(out) < steps:
+        out += [rng.choice(choices)] * rng.choice([1, 1, 2, 3])
+    return out[:steps]
+
+
+def run(steps, ntile, seed, mutate=None, skips=False, max_steps=200000):
     rng = random.Random(seed)
-    cta = FwdCta(steps, ntile, rng, mutate)
+    visible = random_visibility(steps, ntile, rng) if skips else [(True,) * ntile] * steps
+    cta = FwdCta(visible, ntile, rng, mutate)
     roles = {"producer": cta.producer(), "mma": cta.mma()}
     for t in range(ntile):
         roles[f"softmax{t}"] = cta.softmax(t)
@@ -174,12 +199,20 @@ def test_protocol_completes_under_random_interleavings(steps, ntile):
         run(steps, ntile, seed)
 
 
-@pytest.mark.parametrize("mutate", ["no_k_empty_wait", "no_p_full_wait", "s_full_parity"])
-def test_model_sees_protocol_faults(mutate):
+@pytest.mark.parametrize("steps", [1, 2, 3, 4, 7, 12])
+def test_tiles_skipped_for_one_query_tile(steps):
+    for seed in range(150):
+        run(steps, 2, seed, skips=True)
+
+
+@pytest.mark.parametrize("mutate,skips", [("no_k_empty_wait", False), ("no_p_full_wait", False), ("s_full_parity", False),
+                                          ("no_k_empty_wait", True), ("no_p_full_wait", True), ("s_full_parity", True),
+                                          ("s_full_parity_of_list", True), ("p_full_parity_of_list", True)])
+def test_model_sees_protocol_faults(mutate, skips):
     failures = 0
     for seed in range(40):
         try:
-            run(6, 2, seed, mutate)
+            run(6, 2, seed, mutate, skips)
         except AssertionError:
             failures += 1
     assert failures >= 10, f"{mutate}: only {failures} of 40 runs failed"
