@@ -64,8 +64,7 @@ struct BwdParams {
   float scale;
   // Optional, honoured by the tcgen05 kernel only: when dk_out.ptr is set this call is the
   // whole backward for these keys (ring of one) and the kernel stores dK, dV in the input
-  // dtype straight to the result tensors; dk / dv above are then left alone, or hold sums of the
-  // kernel's own (lengths that are not multiples of 128).
+  // dtype straight to the result tensors; dk / dv above are then not touched.
   TensorView dk_out, dv_out;
   // Optional: dk / dv above hold nothing yet and this call defines them (stores instead of
   // read-add-write, zeros for key rows that no query sees), so the caller need not clear them.
@@ -79,6 +78,9 @@ cudaError_t simt_bwd_block(const BwdParams& p, int dtype, cudaStream_t s);
 // Head dims 17 to 128 of the two above.
 cudaError_t simt_wide_fwd(const FwdParams& p, int dtype, cudaStream_t s);
 cudaError_t simt_wide_bwd(const BwdParams& p, int dtype, cudaStream_t s);
+inline bool simt_wide_dims(int dk, int dv) { return (dk > 16 || dv > 16) && dk <= 128 && dv <= 128; }
+// Stream-ordered scratch that simt_bwd_block takes for a block of this shape.
+size_t simt_bwd_scratch_bytes(int b, int h, int lq, int lk, int dk, int dv);
 // out = o / l, L = m + log l (ring.py:134-135).  With o2 != NULL the two carried states are
 // merged first, as one more online-softmax update (ring.py:63-75) would.
 cudaError_t launch_finalize(int b, int h, int lq, int dv, const float* o, const float* m, const float* l,

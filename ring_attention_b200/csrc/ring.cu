@@ -1578,11 +1578,12 @@ int ra_ring_reserve(ra_ring_t* ring, const ra_shape_t* shape, const ra_score_mod
       for (int i = 0; i < kSlots; ++i) RA_CUDA(ring->part[i].reserve(z.dk_b + z.dv_b), "cudaMalloc(part)");
   }
   if (N > 1 && (rc = ensure_shared(ring, msg.total, backward ? z.dk_b + z.dv_b : 0))) return rc;
-  // the block kernels take their tile summaries from a stream-ordered pool that keeps what it
-  // was given: give it this shape's worth now
+  // the block kernels take their tile summaries and the parts of split sums from a stream-ordered pool that
+  // keeps what it was given: give it this shape's worth now (two compute lanes take theirs at the same time)
   void* tmp = nullptr;
-  const size_t meta_bytes = (size_t)shape->b * ((shape->lq + 127) / 128 + (shape->lk + 127) / 128) * sizeof(TileMeta);
-  RA_CUDA(scratch_alloc(&tmp, meta_bytes, ring->push_stream), "scratch pool");
+  size_t scratch = (size_t)shape->b * ((shape->lq + 127) / 128 + (shape->lk + 127) / 128) * sizeof(TileMeta);
+  if (backward) scratch += simt_bwd_scratch_bytes(shape->b, shape->h, shape->lq, shape->lk, shape->dk, shape->dv);
+  RA_CUDA(scratch_alloc(&tmp, N > 1 ? 2 * scratch : scratch, ring->push_stream), "scratch pool");
   RA_CUDA(cudaFreeAsync(tmp, ring->push_stream), "cudaFreeAsync");
   RA_CUDA(cudaStreamSynchronize(ring->push_stream), "cudaStreamSynchronize");
   return 0;

@@ -684,15 +684,12 @@ cudaError_t dispatch_bwd(const BwdParams& p, cudaStream_t s) {
 
 }  // namespace
 
-// Whether simt_wide.cu serves these head dims.
-static bool wide(int dk, int dv) { return (dk > 16 || dv > 16) && dk <= 128 && dv <= 128; }
-
 cudaError_t simt_fwd_block(const FwdParams& p, int dtype, cudaStream_t s) {
-  if (wide(p.dk, p.dv)) return simt_wide_fwd(p, dtype, s);
+  if (simt_wide_dims(p.dk, p.dv)) return simt_wide_fwd(p, dtype, s);
   return dtype == RA_DTYPE_F32 ? dispatch_fwd<float>(p, s) : dispatch_fwd<__nv_bfloat16>(p, s);
 }
 cudaError_t simt_bwd_block(const BwdParams& p, int dtype, cudaStream_t s) {
-  if (wide(p.dk_dim, p.dv_dim)) return simt_wide_bwd(p, dtype, s);
+  if (simt_wide_dims(p.dk_dim, p.dv_dim)) return simt_wide_bwd(p, dtype, s);
   return dtype == RA_DTYPE_F32 ? dispatch_bwd<float>(p, s) : dispatch_bwd<__nv_bfloat16>(p, s);
 }
 

@@ -16,6 +16,7 @@
 #include "common.cuh"
 #include "host_util.h"
 #include "ptx_sm100.cuh"
+#include "tc_common.cuh"
 
 namespace ra {
 
@@ -435,52 +436,76 @@ __global__ void __launch_bounds__(16 * TY, D_PAD == 64 ? 2 : 1) wide_fwd_kernel(
   }
 }
 
-// Adds a thread's R x D_PAD/32 pairs to rows row0 + i of an fp32 [.., rows, dim] accumulator; `atomic`:
-// other CTAs add to the same rows.
+__device__ __forceinline__ bool rows_aligned(const float* base, int dim) {
+  return ((reinterpret_cast<uintptr_t>(base) | (uintptr_t)(dim * 4)) & 15) == 0;
+}
+// Adds x to columns [c, c + 4) of a row of `dim` floats; `vec`: rows are 16-byte aligned; `atomic`: other
+// CTAs add to the same row.
+__device__ __forceinline__ void add4(float* row, int c, int dim, const float (&x)[4], bool vec, bool atomic) {
+  if (vec) {
+    if (c >= dim) return;
+    if (atomic) {
+      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(row + c), "f"(x[0]), "f"(x[1]), "f"(x[2]), "f"(x[3])
+                   : "memory");
+    } else {
+      float4 a = *reinterpret_cast<float4*>(row + c);
+      a.x += x[0], a.y += x[1], a.z += x[2], a.w += x[3];
+      *reinterpret_cast<float4*>(row + c) = a;
+    }
+  } else {
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (c + u < dim) {
+        if (atomic) atomicAdd(row + c + u, x[u]);
+        else row[c + u] += x[u];
+      }
+  }
+}
+
+// Adds a thread's R x D_PAD/32 pairs to rows row0 + i of an fp32 [.., rows, dim] accumulator.
 template <int D_PAD, int R>
 __device__ __forceinline__ void add_rows(float* base, const uint64_t (&v)[R][D_PAD / 32], int row0, int nrows, int dim, int tx,
                                          bool atomic) {
-  const bool vec = ((reinterpret_cast<uintptr_t>(base) | (uintptr_t)(dim * 4)) & 15) == 0;
+  const bool vec = rows_aligned(base, dim);
 #pragma unroll
   for (int i = 0; i < R; ++i) {
     if (row0 + i >= nrows) continue;
-    float* row = base + (int64_t)(row0 + i) * dim;
 #pragma unroll
     for (int cc = 0; cc < D_PAD / 64; ++cc) {
-      const int c = tx * 4 + 64 * cc;
       float x[4];
       unpack2(v[i][2 * cc], x[0], x[1]);
       unpack2(v[i][2 * cc + 1], x[2], x[3]);
-      if (vec) {
-        if (c >= dim) continue;
-        if (atomic) {
-          asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(row + c), "f"(x[0]), "f"(x[1]), "f"(x[2]), "f"(x[3])
-                       : "memory");
-        } else {
-          float4 a = *reinterpret_cast<float4*>(row + c);
-          a.x += x[0], a.y += x[1], a.z += x[2], a.w += x[3];
-          *reinterpret_cast<float4*>(row + c) = a;
-        }
-      } else {
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (c + u < dim) {
-            if (atomic) atomicAdd(row + c + u, x[u]);
-            else row[c + u] += x[u];
-          }
-      }
+      add4(base + (int64_t)(row0 + i) * dim, tx * 4 + 64 * cc, dim, x, vec, atomic);
     }
   }
+}
+
+// One split's dK and dV of a key tile: [dK, dV][64][D_PAD].  `used` (an array behind the parts) says which
+// parts hold anything: a mask leaves some splits without a visible tile.
+template <int D_PAD>
+constexpr int64_t kPartFloats = 2 * BT * D_PAD;
+template <int D_PAD, int R>
+__device__ __forceinline__ void put_rows(float* part, const uint64_t (&v)[R][D_PAD / 32], int row0, int tx) {
+#pragma unroll
+  for (int i = 0; i < R; ++i)
+#pragma unroll
+    for (int cc = 0; cc < D_PAD / 64; ++cc)
+      *reinterpret_cast<ulonglong2*>(part + (row0 + i) * D_PAD + tx * 4 + 64 * cc) =
+          make_ulonglong2(v[i][2 * cc], v[i][2 * cc + 1]);
 }
 
 // ---------------------------------------------------------------------------------------
 // Backward block (ring.py:140-157).  A CTA owns 64 keys and every `splits`-th query tile: a short
 // sequence has too few key tiles for 148 SMs, and the tiles one of them would walk alone are a
-// serial chain.  With one split dK and dV are plain sums, with more they are added atomically (as
-// dQ always is).  The next Q and dO tiles arrive under the dQ product.
+// serial chain.  With one split a CTA adds its dK and dV itself; with more each leaves them in a part of its
+// own and sum_parts_kernel adds the parts in a fixed order, so that repeated calls give the same bits
+// (dQ is added atomically and does not).  Atomic additions of dK and dV instead cost the same; the splits as a
+// cluster with the sums in shared memory held every SM until a tile's slowest split was done (causal 1k, d 128:
+// 206 against 134 us; a window of 125 of 1000 tokens: 279 against 134 us).
+// The next Q and dO tiles arrive under the dQ product.
 // ---------------------------------------------------------------------------------------
 template <typename T, int D_PAD, int TY>
-__global__ void __launch_bounds__(16 * TY, D_PAD == 64 ? 2 : 1) wide_bwd_kernel(const BwdParams p, int splits) {
+__global__ void __launch_bounds__(16 * TY, D_PAD == 64 ? 2 : 1) wide_bwd_kernel(const BwdParams p, int splits, float* parts, int* used) {
   constexpr int P = D_PAD + 4, R = BT / TY, NT = 16 * TY, NO = D_PAD / 32;
   extern __shared__ __align__(16) float smem[];
   float* Qs = smem;
@@ -511,6 +536,7 @@ __global__ void __launch_bounds__(16 * TY, D_PAD == 64 ? 2 : 1) wide_bwd_kernel(
   Stage<T, D_PAD, NT, BT>().whole(Ks, kb, p.k.sl, k0, p.lk, p.dk_dim);
   Stage<T, D_PAD, NT, BT>().whole(Vs, vb, p.v.sl, k0, p.lk, p.dv_dim);
 
+  bool any = false;
   const int n_tiles = (p.lq + BT - 1) / BT;
   for (int base = 0; base < n_tiles; base += kClsTiles) {
     __syncthreads();
@@ -534,6 +560,7 @@ __global__ void __launch_bounds__(16 * TY, D_PAD == 64 ? 2 : 1) wide_bwd_kernel(
     int t = next(0);
     if (t < end) stage_q(t);
     cp_commit();
+    any = any || t < end;
     while (t < end) {
       const int q0 = (base + t) * BT, tn = next(t + 1);
       if (tid < BT) {
@@ -589,8 +616,58 @@ __global__ void __launch_bounds__(16 * TY, D_PAD == 64 ? 2 : 1) wide_bwd_kernel(
     }
   }
   cp_wait<0>();
-  add_rows<D_PAD, R>(p.dk + krow_base * p.dk_dim, dk_acc, k0 + ty * R, p.lk, p.dk_dim, tx, splits > 1);
-  add_rows<D_PAD, R>(p.dv + krow_base * p.dv_dim, dv_acc, k0 + ty * R, p.lk, p.dv_dim, tx, splits > 1);
+  if (splits == 1) {
+    add_rows<D_PAD, R>(p.dk + krow_base * p.dk_dim, dk_acc, k0 + ty * R, p.lk, p.dk_dim, tx, false);
+    add_rows<D_PAD, R>(p.dv + krow_base * p.dv_dim, dv_acc, k0 + ty * R, p.lk, p.dv_dim, tx, false);
+    return;
+  }
+  const int64_t part = ((int64_t)bb * p.h + hh) * gridDim.x + blockIdx.x;
+  if (tid == 0) used[part] = any;
+  if (!any) return;
+  put_rows<D_PAD, R>(parts + part * kPartFloats<D_PAD>, dk_acc, ty * R, tx);
+  put_rows<D_PAD, R>(parts + part * kPartFloats<D_PAD> + BT * D_PAD, dv_acc, ty * R, tx);
+}
+
+// dK, dV += the parts of a key tile.  Four groups of 64 threads add every fourth part each and meet in shared memory:
+// an order that depends on the number of splits alone.  blockIdx: key tile, 64 of its 16-byte chunks, (batch, head).
+template <int D_PAD>
+__global__ void __launch_bounds__(256) sum_parts_kernel(const BwdParams p, int splits, const float* __restrict__ parts,
+                                                        const int* __restrict__ used) {
+  __shared__ float4 sums[4][64];
+  const int k0 = blockIdx.x * BT, i = threadIdx.x & 63, g = threadIdx.x >> 6;
+  const int64_t bh = blockIdx.z, first = (bh * gridDim.x + blockIdx.x) * splits;
+  const int e = blockIdx.y * 64 + i;  // chunk of [dK, dV][64][D_PAD / 4]
+  const float* from = parts + first * kPartFloats<D_PAD> + e * 4;
+  float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+  for (int k = g; k < splits; k += 4)
+    if (used[first + k]) {
+      const float4 v = *reinterpret_cast<const float4*>(from + k * kPartFloats<D_PAD>);
+      x.x += v.x, x.y += v.y, x.z += v.z, x.w += v.w;
+    }
+  sums[g][i] = x;
+  __syncthreads();
+  const int which = e / (BT * D_PAD / 4), r = e / (D_PAD / 4) % BT, c = e % (D_PAD / 4) * 4;
+  const int dim = which ? p.dv_dim : p.dk_dim;
+  if (g || k0 + r >= p.lk || c >= dim) return;
+  float y[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) y[0] += sums[j][i].x, y[1] += sums[j][i].y, y[2] += sums[j][i].z, y[3] += sums[j][i].w;
+  float* base = (which ? p.dv : p.dk) + bh * p.lk * dim;
+  add4(base + (int64_t)(k0 + r) * dim, c, dim, y, rows_aligned(base, dim), false);
+}
+
+// Query splits of a backward: until there are about four CTAs per SM, each with a query tile of its own to look
+// at (a mask may leave some without a visible one).
+int bwd_splits(int b, int h, int lq, int lk) {
+  const int64_t ctas = (int64_t)((lk + BT - 1) / BT) * h * b, q_tiles = (lq + BT - 1) / BT;
+  int64_t splits = (4 * 148 + ctas - 1) / ctas;
+  if (splits > q_tiles) splits = q_tiles;
+  return splits < 1 ? 1 : (int)splits;
+}
+size_t bwd_parts(int b, int h, int lq, int lk) {
+  const int splits = bwd_splits(b, h, lq, lk);
+  return splits == 1 ? 0 : (size_t)((lk + BT - 1) / BT) * h * b * splits;
 }
 
 template <typename T, int D_PAD, int R, int TY>
@@ -611,14 +688,32 @@ cudaError_t launch_bwd(const BwdParams& p, cudaStream_t s) {
   auto kern = wide_bwd_kernel<T, D_PAD, TY>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  // query splits: until about four CTAs per SM, but no CTA without a tile
-  const int64_t ctas = (int64_t)((p.lk + BT - 1) / BT) * p.h * p.b, q_tiles = (p.lq + BT - 1) / BT;
-  int64_t splits = (4 * 148 + ctas - 1) / ctas;
-  if (splits > q_tiles) splits = q_tiles;
-  if (splits < 1) splits = 1;
-  kern<<<dim3((unsigned)((p.lk + BT - 1) / BT * splits), p.h, p.b), 16 * TY, smem, s>>>(p, (int)splits);
+  const unsigned k_tiles = (p.lk + BT - 1) / BT;
+  int splits = bwd_splits(p.b, p.h, p.lq, p.lk);
+  float* parts = nullptr;
+  int* used = nullptr;
+  if (splits > 1) {
+    const size_t n = bwd_parts(p.b, p.h, p.lq, p.lk);
+    if (scratch_alloc((void**)&parts, n * (kPartFloats<D_PAD> * sizeof(float) + sizeof(int)), s) == cudaSuccess) {
+      used = reinterpret_cast<int*>(parts + n * kPartFloats<D_PAD>);
+    } else {  // no memory for the parts: whole key tiles, which need none
+      cudaGetLastError();
+      parts = nullptr;
+      splits = 1;
+    }
+  }
+  kern<<<dim3(k_tiles * splits, p.h, p.b), 16 * TY, smem, s>>>(p, splits, parts, used);
   count_launch();
-  return cudaGetLastError();
+  e = cudaGetLastError();
+  if (parts) {
+    if (e == cudaSuccess) {
+      sum_parts_kernel<D_PAD><<<dim3(k_tiles, kPartFloats<D_PAD> / 4 / 64, p.b * p.h), 256, 0, s>>>(p, splits, parts, used);
+      count_launch();
+      e = cudaGetLastError();
+    }
+    cudaFreeAsync(parts, s);
+  }
+  return e;
 }
 
 template <typename T>
@@ -644,6 +739,11 @@ cudaError_t dispatch_bwd(const BwdParams& p, cudaStream_t s) {
 
 cudaError_t simt_wide_fwd(const FwdParams& p, int dtype, cudaStream_t s) {
   return dtype == RA_DTYPE_F32 ? dispatch_fwd<float>(p, s) : dispatch_fwd<__nv_bfloat16>(p, s);
+}
+size_t simt_bwd_scratch_bytes(int b, int h, int lq, int lk, int dk, int dv) {
+  if (!simt_wide_dims(dk, dv)) return 0;
+  const size_t floats = dk > 64 || dv > 64 ? kPartFloats<128> : kPartFloats<64>;
+  return bwd_parts(b, h, lq, lk) * (floats * sizeof(float) + sizeof(int));
 }
 cudaError_t simt_wide_bwd(const BwdParams& p, int dtype, cudaStream_t s) {
   return dtype == RA_DTYPE_F32 ? dispatch_bwd<float>(p, s) : dispatch_bwd<__nv_bfloat16>(p, s);

@@ -1,6 +1,6 @@
 """What the CUDA-core kernels' routing by head dim owes its callers: a call pays for its own head dims and
 types and not for a larger template's (ratios of device times of two calls of one process, far from what
-a wrong route shows)."""
+a wrong route shows), and dK, dV of repeated calls are the same bits."""
 import pytest
 import torch
 
@@ -64,3 +64,24 @@ def test_those_head_dims_against_the_oracle(dk, dv):
     check_close(out, O.mha(q, k, v), torch.float32, "out")
     for name, got, want in zip(("dq", "dk", "dv"), grads, O.mha_grads(q, k, v, do)):
         check_close(got, want, torch.float32, name, 2e-5)
+
+
+@pytest.mark.parametrize("b,h,lq,lk,d,dtype,mask", [
+    (1, 4, 1024, 1024, 64, torch.float32, True), (2, 4, 777, 1000, 64, torch.float32, False),
+    (1, 2, 300, 500, 33, torch.float32, False), (1, 4, 1000, 1000, 128, torch.float32, True),
+    (1, 4, 1000, 1000, 96, torch.bfloat16, True), (1, 1, 8192, 64, 64, torch.float32, False)])
+def test_repeated_calls_repeat_dk_and_dv(b, h, lq, lk, d, dtype, mask):
+    """Few key tiles: the query range is split over CTAs, whose sums are added in a fixed order."""
+    q, k, v = _qkv(b, h, max(lq, lk), d, d, dtype)
+    t = [x[:, :n].contiguous().requires_grad_(True) for x, n in ((q, lq), (k, lk), (v, lk))]
+    do = torch.randn_like(t[0])
+    kw = {}
+    if mask:
+        pos = torch.arange(lq, dtype=torch.int32, device="cuda").expand(b, lq).contiguous()
+        kw = dict(bias_fn=ra().ScoreMod(causal=True, window=lq // 3), bias_q_kwargs={"q_positions": pos},
+                  bias_kv_kwargs={"kv_positions": pos})
+    out = ra().ring_attention(*t, "sp", block_impl="simt", **kw)
+    first = torch.autograd.grad(out, t, do, retain_graph=True)
+    for _ in range(5):
+        again = torch.autograd.grad(out, t, do, retain_graph=True)
+        assert torch.equal(first[1], again[1]) and torch.equal(first[2], again[2])
