@@ -195,8 +195,10 @@ def _dense_mod(bias: Optional[torch.Tensor], b: int, h: int, lq: int, lk: int):
         bias = bias[:, None]
     if bias.shape[0] != b or bias.shape[1] not in (1, h) or bias.shape[2] != lq or bias.shape[3] != lk:
         raise ValueError(f"bias shape {tuple(bias.shape)} does not match [b={b}, h={h} or 1, {lq}, {lk}]")
-    # The kernels read any batch, head and row strides (0 for a broadcast axis).  A view is copied only
-    # where its rows are not consecutive floats on 16-byte boundaries.
+    # The kernels read any batch, head and row strides (0 for a broadcast axis).  A view whose rows are not
+    # consecutive floats on 16-byte boundaries is copied.  A contiguous tensor stays as it is wherever its base
+    # lies: off 16 bytes the CUDA-core kernels read it (copying it would move bf16 calls to the tensor cores, which
+    # hold P in fewer bits).
     strides = [0 if bias.shape[i] == 1 else bias.stride(i) for i in range(3)]
     if (bias.stride(3) != 1 and lk > 1) or bias.data_ptr() % 16 or any(s % 4 for s in strides):
         bias = bias.contiguous()
