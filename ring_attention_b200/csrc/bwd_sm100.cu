@@ -58,8 +58,11 @@ constexpr int kRegsCompute = 152, kRegsDrain = 152, kRegsOther = 56;
 // run on, round to nearest, so dK and dV move to fp32 sums in global memory after this many query tiles: p.dk and
 // p.dv, where a key tile's n rows are held as [D / 4][n] 16-byte chunks, so that a warp's accesses are contiguous.
 // 20001 causal tokens, d 128: relative error of dK 1.6640e-3 without that, 1.6625e-3 with it and on the CUDA cores;
-// 3001 causal, b 2, h 16: 467 -> 486 us.
+// 3001 causal, b 2, h 16: 470 -> 485 us.
+// A call with no more tiles than that never moves anything and takes the form without the code for it (cross
+// attention 448 x 1500, b 8, h 16, d 64: 264 -> 255 us).
 constexpr int kFlushTiles = 16;
+enum Ragged { kAligned = 0, kRaggedShort, kRaggedLong };
 
 __host__ __device__ constexpr int bwd_do_stages(int d, bool ragged) { return ragged && d == 128 ? 1 : 2; }
 
@@ -88,9 +91,10 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint
       : "memory");
 }
 
-template <int D, bool RAGGED>
+template <int D, int RAGGED>
 __global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_constant__ BwdTcParams P) {
   constexpr int PRODUCER_WARP = 12, MMA_WARP = 13;
+  constexpr bool MOVES = RAGGED == kRaggedLong;  // dK and dV move out every kFlushTiles tiles
   // Head dim 64 leaves tensor memory for columns of dQ^T's own: dP^T of the next tile need not wait
   // until dQ^T has been drained.  It is then issued before the MMAs that read dS^T, so dS^T has two stages.
   // Unmasked 8k tokens, d 64: 3.25 -> 2.40 ms (with dQ formed untransposed, drained by the compute
@@ -397,7 +401,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_con
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk)
               mma_ss_warp(tmem_dK, desc_from_lo(a0 + km_off(kk)), desc_from_lo(b0 + mn_off(kk)), idesc_dv,
-                     (RAGGED ? n % kFlushTiles != 0 : n > 0) || kk > 0);
+                     (MOVES ? n % kFlushTiles != 0 : n > 0) || kk > 0);
             if constexpr (RAGGED) {
 #pragma unroll
               for (int kk = 0; kk < 8; ++kk)
@@ -406,7 +410,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_con
           }
           tc_commit_warp(&bars[Q_EMPTY0 + s]);
           if (!has_next) break;
-          const bool flush = RAGGED && (n + 1) % kFlushTiles == 0;  // dV and dK start afresh with tile n + 1
+          const bool flush = MOVES && (n + 1) % kFlushTiles == 0;  // dV and dK start afresh with tile n + 1
           if (flush) tc_commit_warp(&bars[ACC_FULL]);
           if constexpr (!SEP_DQ) {
             if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[DQ_DRAINED], par, abort_flag, P.status, kStBwdMma)))) break;
@@ -455,7 +459,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_con
         if (!RAGGED || c < q_left)
           asm volatile("red.global.add.f32 [%0], %1;" ::"l"(base + c * D), "f"(__uint_as_float(dv[c >> 5][c & 31])) : "memory");
       i = next_active(win, i + 1) & kTileIdx;
-      if constexpr (RAGGED) {
+      if constexpr (MOVES) {
         if ((n + 1) % kFlushTiles == 0 && i < P.n_q_tiles) {
           // dV, dK of the last kFlushTiles tiles to this thread's key row of the fp32 sums (nobody else adds to it)
           if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[ACC_FULL], ((n + 1) / kFlushTiles - 1) & 1, abort_flag, P.status, kStBwdCompute)))) break;
@@ -664,9 +668,9 @@ __global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_con
     }
     const int n = k > 0 ? 1 : 0;
     // ---- epilogue: dK, dV of this K/V tile
-    constexpr int kSumChunks = RAGGED ? D / 8 : 1;
-    float4 sum[kSumChunks];  // RAGGED: this row's half of the sum of earlier tiles
-    const int flushes = RAGGED && k > 0 ? (k - 1) / kFlushTiles : 0;
+    constexpr int kSumChunks = MOVES ? D / 8 : 1;
+    float4 sum[kSumChunks];  // MOVES: this row's half of the sum of earlier tiles
+    const int flushes = MOVES && k > 0 ? (k - 1) / kFlushTiles : 0;
     auto load_sum = [&](const float* sums) {
       const int rows = min(kTileRows, p.lk - kt * kTileRows);
       const float* from = sums + (((int64_t)bb * p.h + hh) * p.lk + kt * kTileRows) * D + r * 4 + g * (D / 2) * rows;
@@ -674,7 +678,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_con
       for (int j = 0; j < kSumChunks; ++j)
         sum[j] = flushes > 0 && row_valid ? __ldcg(reinterpret_cast<const float4*>(from + 4 * j * rows)) : make_float4(0.f, 0.f, 0.f, 0.f);
     };
-    if constexpr (RAGGED) {  // dK's is on its way while the last MMAs run
+    if constexpr (MOVES) {  // dK's is on its way while the last MMAs run
       if (ok && flushes > 0) ok = __all_sync(0xffffffffu, mbar_wait(&bars[ACC_FLUSHED], (flushes - 1) & 1, abort_flag, P.status, kStBwdCompute));
       if (ok) load_sum(p.dk);
     }
@@ -684,11 +688,11 @@ __global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_con
       auto put = [&](uint32_t tmem, const TensorView& out) {
         __nv_bfloat16* to = (__nv_bfloat16*)out.ptr + (int64_t)bb * out.sb + (int64_t)kv_row * out.sl + (int64_t)hh * out.sh + g * (D / 2);
 #pragma unroll
-        for (int j = 0; j + 1 < kSumChunks; j += 2) {
+        for (int j = 0; j < D / 8; j += 2) {
           uint32_t a[8];
           tmem_ld8(tmem + lane_off + g * (D / 2) + j * 4, a);
           tc_wait_ld();
-          const float4 x = sum[j], y = sum[j + 1];
+          const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), x = MOVES ? sum[MOVES ? j : 0] : zero, y = MOVES ? sum[MOVES ? j + 1 : 0] : zero;
           uint4 w;
           w.x = pack_bf16(x.x + __uint_as_float(a[0]), x.y + __uint_as_float(a[1]));
           w.y = pack_bf16(x.z + __uint_as_float(a[2]), x.w + __uint_as_float(a[3]));
@@ -698,7 +702,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_con
         }
       };
       put(tmem_dK, p.dk_out);
-      load_sum(p.dv);
+      if constexpr (MOVES) load_sum(p.dv);
       put(tmem_dV, p.dv_out);
     } else if (!RAGGED && ok && n > 0) {
       tc_fence_after();
@@ -791,7 +795,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) tc_bwd_kernel(const __grid_con
   }
 }
 
-template <int D, bool RAGGED>
+template <int D, int RAGGED>
 cudaError_t launch_bwd(const BwdTcParams& P, cudaStream_t s) {
   constexpr size_t kSmem = (4 + bwd_do_stages(D, RAGGED)) * kTileRows * D * 2 +
                            (D == 64 ? 2 : 1) * (RAGGED ? 2 : 1) * kTileRows * kTileRows * 2 + 4 * kTileRows * 4 + NUM_BARS * 8 + 64;
@@ -890,8 +894,9 @@ cudaError_t tc_bwd_block(const BwdParams& p, cudaStream_t s) {
   }
   const bool ragged = p.lq % kTileRows || p.lk % kTileRows;
   if (e == cudaSuccess) {
-    if (ragged) e = p.dk_dim == 128 ? launch_bwd<128, true>(P, s) : launch_bwd<64, true>(P, s);
-    else e = p.dk_dim == 128 ? launch_bwd<128, false>(P, s) : launch_bwd<64, false>(P, s);
+    if (!ragged) e = p.dk_dim == 128 ? launch_bwd<128, kAligned>(P, s) : launch_bwd<64, kAligned>(P, s);
+    else if (P.n_q_tiles <= kFlushTiles) e = p.dk_dim == 128 ? launch_bwd<128, kRaggedShort>(P, s) : launch_bwd<64, kRaggedShort>(P, s);
+    else e = p.dk_dim == 128 ? launch_bwd<128, kRaggedLong>(P, s) : launch_bwd<64, kRaggedLong>(P, s);
   }
   if (meta) cudaFreeAsync(meta, s);  // stream-ordered: after the kernels above, also when one failed to launch
   if (terms) cudaFreeAsync(terms, s);

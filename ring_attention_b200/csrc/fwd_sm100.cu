@@ -19,8 +19,8 @@
 // stored.  These calls used to run on the CUDA cores with P in fp32, so here P keeps 16 bits: it goes
 // to TMEM as two bf16 halves (hi in the first, lo in the second half of S's columns) and PV runs twice;
 // every exponential is ex2.  What bounds it is the same softmax path plus 1.5 times the MMAs.  Causal
-// 3001 tokens, b 2, h 16, d 128, forward + backward: 15.6 -> 0.64 ms; 448 x 1500, b 8, h 16, d 64: 4.0 ->
-// 0.35 ms.  Relative error against 64 bits from 333 to 20001 tokens (the results' bf16 rounding): out 1.57e-3 to
+// 3001 tokens, b 2, h 16, d 128, forward + backward: 15.6 -> 0.63 ms; 448 x 1500, b 8, h 16, d 64: 4.0 ->
+// 0.33 ms.  Relative error against 64 bits from 333 to 20001 tokens (the results' bf16 rounding): out 1.57e-3 to
 // 1.66e-3, gradients 1.64e-3 to 1.67e-3, the same to four digits as on the CUDA cores.
 // TMEM columns: S0 [0,128) S1 [128,256) O0 [256,256+D) O1 [256+D,256+2D).
 #include <cstdio>
@@ -49,8 +49,11 @@ constexpr float kRescaleThreshold = 8.0f;  // log2 units: P stays below 2^8
 // round to nearest, so O moves to an fp32 sum in global memory after this many tiles: p.o, where a query
 // tile's n rows are held as [D / 4][n] 16-byte chunks, so that a warp's accesses are contiguous.  9842 tokens, no
 // mask, d 128: out comes 2.3e-5 of itself too small without that, 1.0e-5 with it (CUDA cores 0.4e-5; the bf16
-// rounding hides factors below about 1e-5); 5454 tokens, b 2, h 8: 367 -> 394 us.
+// rounding hides factors below about 1e-5); 5454 tokens, b 2, h 8: 366 -> 391 us.
+// A call with no more tiles than that never moves anything and takes the form without the code for it (cross
+// attention 448 x 1500, b 8, h 16, d 64: 80 -> 77 us).
 constexpr int kFlushTiles = 32;
+enum Ragged { kAligned = 0, kRaggedShort, kRaggedLong };
 // Of every 16 column pairs of the softmax, how many get their exponentials from the polynomial
 // on the FMA pipe (the others use ex2 on the special-function unit).  Measured per value, two to three
 // alternating runs each, which agree to 0.5 % (us; SM clock 1965 MHz unless noted):
@@ -80,7 +83,7 @@ enum Bar {
   S_FULL0, S_FULL1, P_FULL0, P_FULL1, O_FULL, NUM_BARS
 };
 
-// RAGGED: a row's O moves from tensor memory to its fp32 sum (chunk j of the row at sums + j * pitch), which was
+// A row's O moves from tensor memory to its fp32 sum (chunk j of the row at sums + j * pitch), which was
 // scaled by `alpha` since the last move.  The warp calls it together; kept out of line, because the loop that
 // calls it is short of registers.
 template <int D>
@@ -113,11 +116,12 @@ __device__ __noinline__ void move_o(uint32_t tmem, float* sums, int pitch, bool 
 // PLAIN: a call without score-mods.  Its loop holds no mask code; at head dim 64, where the softmax warps are what
 // the kernel waits for, carrying that code cost 8 % (6144 tokens, b 1, h 16: 260 -> 238 us; at head dim 128 the
 // masked form serves such calls, 309 against 302 us).
-template <int D, bool RAGGED, bool PLAIN = false>
+template <int D, int RAGGED, bool PLAIN = false>
 __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_constant__ FwdTcParams P) {
   constexpr int TILE_BYTES = kTileRows * D * 2;
   constexpr int PANELS = D / 64;           // 64-element (128-byte) panels per row
   constexpr int PANEL_BYTES = kTileRows * 128;
+  constexpr bool MOVES = RAGGED == kRaggedLong;  // O moves out every kFlushTiles tiles
   constexpr int kPolyPairs = RAGGED ? 0 : poly_pairs(D, PLAIN);
   // Which form of the wait for S (below): a vote costs head dim 128 nothing (32k causal tokens 8345 us, 8418 without
   // it), head dim 64 and the ragged forms 1 to 6 % (8k causal, d 64: 438 against 425 us; 3001 causal, d 128: 152, 145).
@@ -297,7 +301,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
           if (cur & (kVisible << t)) {
             if (!(ok = __all_sync(0xffffffffu, mbar_wait(&bars[P_FULL0 + t], done[t] & 1, abort_flag, P.status, kStFwdMma)))) break;
             tc_fence_after();
-            issue_pv(t, s, RAGGED ? done[t] % kFlushTiles == 0 : done[t] == 0);
+            issue_pv(t, s, MOVES ? done[t] % kFlushTiles == 0 : done[t] == 0);
             ++done[t];
           }
           if (t == ntile - 1) tc_commit_warp(&bars[V_EMPTY0 + s]);
@@ -340,7 +344,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
     const bool has_pos = !PLAIN && p.mod.kv_pos != nullptr;
     int32_t k0_next = (has_pos && count > 0) ? p.mod.kv_pos[(int64_t)bb * p.lk + (int64_t)(list[0] & kTileIdx) * kTileRows] : 0;
     int done = 0;  // K/V tiles this query tile has been through
-    // RAGGED: once more than kFlushTiles tiles are done p.o holds the sum of earlier ones, to be multiplied by
+    // MOVES: once more than kFlushTiles tiles are done p.o holds the sum of earlier ones, to be multiplied by
     // alpha_total; this row's chunk j is at o_sum() + j * o_pitch()
     auto o_pitch = [&]() { return 4 * min(kTileRows, p.lq - (qt0 + t) * kTileRows); };
     auto o_sum = [&]() { return p.o + (((int64_t)bb * p.h + hh) * p.lq + (qt0 + t) * kTileRows) * D + row_in_tile * 4; };
@@ -371,7 +375,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
         mbar_wait(&bars[S_FULL0 + t], done & 1, abort_flag, P.status, kStFwdSoftmax);
       }
       tc_fence_after();
-      if constexpr (RAGGED) {
+      if constexpr (MOVES) {
         // P V of the tiles before is complete (S of this one was issued behind it) and the next one starts O afresh
         if (done > 0 && done % kFlushTiles == 0) {
           move_o<D>(tmem_O[t] + lane_off, o_sum(), o_pitch(), row_valid, done > kFlushTiles, alpha_total);
@@ -426,7 +430,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
         m_ref = m_new;
         l_run *= alpha;
         alpha_total *= alpha;
-        if (RAGGED ? done % kFlushTiles != 0 : done > 0) {  // O of this tile holds the sum over the tiles before this one
+        if (MOVES ? done % kFlushTiles != 0 : done > 0) {  // O of this tile holds the sum over the tiles before this one
 #pragma unroll 1
           for (int c = 0; c < D / 16; ++c) {
             uint32_t o[16];
@@ -479,9 +483,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
 
     // Epilogue: fold in the carried state of earlier ring steps, bring (o, m, l) to the
     // exact running max, store.
-    constexpr int kSumChunks = RAGGED ? D / 4 : 1;
-    float4 sum[kSumChunks];  // RAGGED: the sum of earlier tiles, on its way while the last MMAs run
-    if constexpr (RAGGED) {
+    constexpr int kSumChunks = MOVES ? D / 4 : 1;
+    float4 sum[kSumChunks];  // MOVES: the sum of earlier tiles, on its way while the last MMAs run
+    if constexpr (MOVES) {
 #pragma unroll
       for (int j = 0; j < kSumChunks; ++j)
         sum[j] = done > kFlushTiles && row_valid ? __ldcg(reinterpret_cast<const float4*>(o_sum() + j * o_pitch()))
@@ -492,7 +496,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
       tc_fence_after();
       const float beta = (m_ref == -INFINITY) ? 1.f : ex2(m_ref - m_true);
       // a ragged call is the whole attention: no carried state but its own sum of earlier tiles, results go out
-      const bool first = RAGGED ? done <= kFlushTiles : p.first != 0;
+      const bool first = MOVES ? done <= kFlushTiles : (RAGGED || p.first);
       const float in_scale = first ? 0.f : alpha_total * beta;
       float* o_row = p.o + state_row * D;
       const bool finalize = RAGGED || p.final_out.ptr != nullptr;
@@ -501,7 +505,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
       __nv_bfloat16* out_row = finalize ? (__nv_bfloat16*)p.final_out.ptr + (int64_t)bb * p.final_out.sb +
                                               (int64_t)q_row * p.final_out.sl + (int64_t)hh * p.final_out.sh
                                         : nullptr;
-#pragma unroll (RAGGED ? D / 8 : 1)
+#pragma unroll (MOVES ? D / 8 : 1)
       for (int c = 0; c < D / 8; ++c) {
         uint32_t o[8];
         if (done > 0) {
@@ -515,7 +519,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) tc_fwd_kernel(const __grid_con
 #pragma unroll
         for (int e = 0; e < 8; e += 4) {
           float4 prev = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (RAGGED) prev = sum[RAGGED ? c * 2 + e / 4 : 0];
+          if (MOVES) prev = sum[MOVES ? c * 2 + e / 4 : 0];
           else if (!first) prev = *reinterpret_cast<const float4*>(o_row + c * 8 + e);
           val[e] = __uint_as_float(o[e]) * beta + prev.x * in_scale;
           val[e + 1] = __uint_as_float(o[e + 1]) * beta + prev.y * in_scale;
@@ -643,7 +647,7 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-template <int D, bool RAGGED, bool PLAIN = false>
+template <int D, int RAGGED, bool PLAIN = false>
 cudaError_t launch_fwd(const FwdTcParams& P, cudaStream_t s) {
   constexpr size_t kSmem = 6 * kTileRows * D * 2 + kMaxTiles * 5 + NUM_BARS * 8 + 64 + 1024;
   constexpr size_t kRequest = kSmem < 120 * 1024 ? 120 * 1024 : kSmem;  // one CTA per SM: it owns all of TMEM
@@ -658,9 +662,9 @@ cudaError_t launch_fwd(const FwdTcParams& P, cudaStream_t s) {
 
 // Lengths that are multiples of 128.
 cudaError_t launch_fwd_aligned(const FwdTcParams& P, cudaStream_t s) {
-  if (P.p.dk == 128) return launch_fwd<128, false>(P, s);
+  if (P.p.dk == 128) return launch_fwd<128, kAligned>(P, s);
   const bool plain = (P.p.mod.kinds & (kMetaKinds | RA_MOD_DENSE)) == 0;
-  return plain ? launch_fwd<64, false, true>(P, s) : launch_fwd<64, false>(P, s);
+  return plain ? launch_fwd<64, kAligned, true>(P, s) : launch_fwd<64, kAligned>(P, s);
 }
 
 }  // namespace
@@ -797,8 +801,9 @@ cudaError_t tc_fwd_block(const FwdParams& p, cudaStream_t s) {
   }
   const bool ragged = p.lq % kTileRows || p.lk % kTileRows;
   if (e == cudaSuccess) {
-    if (ragged) e = p.dk == 128 ? launch_fwd<128, true>(P, s) : launch_fwd<64, true>(P, s);
-    else e = launch_fwd_aligned(P, s);
+    if (!ragged) e = launch_fwd_aligned(P, s);
+    else if (P.n_kv_tiles <= kFlushTiles) e = p.dk == 128 ? launch_fwd<128, kRaggedShort>(P, s) : launch_fwd<64, kRaggedShort>(P, s);
+    else e = p.dk == 128 ? launch_fwd<128, kRaggedLong>(P, s) : launch_fwd<64, kRaggedLong>(P, s);
   }
   if (meta) cudaFreeAsync(meta, s);  // stream-ordered: after the kernels above, also when one failed to launch
   return e;

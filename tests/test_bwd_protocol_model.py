@@ -18,7 +18,7 @@ The kernel has three forms, and the model has them as `Form`:
 * head dim 128: dQ^T overlays dP^T, so dP(n+1) is issued behind dQ(n), dK(n) and the drain of dQ(n);
   one dS buffer, two dO stages;
 * head dim 128 with ragged lengths: the same with one dO stage (a second dS tile has its room); every few
-  tiles the drain warpgroup moves dK and dV out and the MMAs start them afresh;
+  tiles the drain warpgroup moves dK and dV out and the MMAs start them afresh (not in short calls);
 * head dim 64: dQ^T has columns of its own, dP(n+1) is issued before dQ(n), dS has two stages, and the
   drain of dQ(n-1) is waited for before dQ(n); with ragged lengths dK and dV are moved out as well.
 The other buffers: shared memory K/V and Q[2] (with the per-row terms of the stage); tensor memory
@@ -38,6 +38,7 @@ import pytest
 # meet it often)
 Form = namedtuple("Form", "sep_dq ds_stages do_stages flush")
 FORMS = {"head_dim_128": Form(False, 1, 2, 0), "head_dim_128_ragged": Form(False, 1, 1, 2),
+         "head_dim_128_ragged_short": Form(False, 1, 1, 0),
          "head_dim_64": Form(True, 2, 2, 0), "head_dim_64_ragged": Form(True, 2, 2, 2)}
 
 

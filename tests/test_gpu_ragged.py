@@ -52,7 +52,9 @@ def _agree(got, want, what):
     assert not (bad & ~want.isnan()).any(), f"{what}: {(got - want).abs().nan_to_num().max():.3e}"
 
 
-SIZES = [(1, 1), (1, 300), (300, 1), (127, 129), (129, 127), (128, 200), (200, 128), (255, 385), (448, 1500), (1025, 1025)]
+SIZES = [(1, 1), (1, 300), (300, 1), (127, 129), (129, 127), (128, 200), (200, 128), (255, 385), (448, 1500), (1025, 1025),
+         # tiles in a row at which sums start to move out: dK and dV from 17 query tiles, O from 33 key tiles
+         (2048, 100), (2049, 100), (4100, 70), (100, 4096), (70, 4097), (70, 8200)]
 
 
 @pytest.mark.parametrize("d", [64, 128])
