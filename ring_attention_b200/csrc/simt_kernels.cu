@@ -2,9 +2,9 @@
 // attention), any score-mod including a dense bias tile, fp32 or bf16 inputs with all
 // arithmetic in fp32.  They are the exact path (1e-5 against an fp64 restatement of
 // ring_attention/ring.py:58-76 and :140-157) and serve every shape the tcgen05 kernels
-// do not take.  The kernels of this file serve head dims up to 16 (a quarter of the padded
-// columns of the wide kernels) and above 128 (whose tiles do not fit in shared memory whole);
-// the ones between go to simt_wide.cu.
+// do not take.  The kernels of this file serve calls with both head dims up to 16 (a quarter of
+// the padded columns of the wide kernels) or either above 128 (whose tiles do not fit in shared
+// memory whole); the ones between go to simt_wide.cu.
 #include <math.h>
 
 #include "common.cuh"

@@ -7,10 +7,10 @@
 // reads its operands as 16-byte vectors in products on packed fp32 pairs,
 // and tiles are classified from position / segment ranges, so that only tiles which really mix
 // visible and masked pairs look at pairs.
-// Measured (device time of the whole pass, before -> now): 2048 x 2048, b 2, h 4, d 64, no mask:
-// forward 529 -> 320 us, backward 1125 -> 710 us; d 128: 933 -> 601, 2977 -> 1283 us; causal 1024,
-// b 1, h 4, d 64: 228 -> 83, 423 -> 105 us.  What bounds it now is the FMA pipe together with the
-// shared-memory reads (25 to 33 of 74 TFLOP/s): one or two warps per scheduler do not hide them all.
+// Measured (device time, general kernels -> these): 1500 x 1500, b 2, h 4, fp32, no mask: d 64 forward
+// 372 -> 245 us, backward 830 -> 399 us; d 128: 643 -> 456, 2088 -> 775 us; causal 1024, b 1, h 4, d 64:
+// 177 -> 80, 387 -> 95 us.  What bounds it now is the FMA pipe together with the shared-memory reads (25 to
+// 33 of 74 TFLOP/s): two (head dims above 64) to four warps per scheduler do not hide them all.
 #include <math.h>
 
 #include "common.cuh"

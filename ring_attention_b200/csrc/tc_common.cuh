@@ -123,7 +123,8 @@ __device__ __forceinline__ void visible_columns(uint32_t (&vis)[kWords], uint32_
 
 // Adds a per-pair bias to raw (unscaled) scores that sit in TMEM, in place: this thread's TMEM
 // lane, `ncols` columns (a multiple of 16) from `taddr`.  Two biases come this way: ALiBi over
-// columns at scattered positions (over contiguous ones it is two FMAs in the kernels' loops), and
+// columns at scattered positions (over contiguous ones it is FMAs in the kernels' loops, one per score in
+// the forward and two in the backward), and
 // a dense bias tile (RA_MOD_DENSE: the materialised bias_fn result of ring.py:60-61).  Both are
 // added divided by the softmax scale, so that the main loops, which multiply by the scale, see
 // exactly scale * s + bias.  A rolled loop on purpose: the main loops stay small enough for the
